@@ -11,6 +11,12 @@
 //   X_rr^-1  by Gauss-Jordan elimination with partial pivoting (kept: the
 //            solve sweeps multiply by it instead of solving with LU factors)
 //   U        = X_rr^{-1} K_r_sn,  L = K_sn_r X_rr^{-1}   (GEMMs)
+//   L       += (K_sn_r - L X_rr) X_rr^{-1}   (reference mode: a product with
+//            the inverse from the right leaves a residual of cond(X_rr) eps,
+//            where the reference's triangular solves leave eps; on the
+//            4,096-node circle at id_tol 1e-13 the solution's error against
+//            the analytic one is 1e-12 without this correction, 1e-14 with
+//            it.  A preconditioner does not need it)
 //   acc      = update(s, s) + L K_r_sn      (what the ancestors subtract)
 // The reference re-searches every compressed descendant's skeleton inside
 // the parent's index list (skel_factorization.cpp:246-294); here each box
@@ -52,6 +58,7 @@ __global__ void __launch_bounds__(kDecThreads) decouple_kernel(DecParams P) {
   double* L = tk.L;
   double* U = tk.U;
   double* X = tk.X;
+  double* Xk = tk.X0 ? tk.X0 : X;  // X_rr itself, kept where L is corrected
   double* acc = tk.acc;
   int* piv = tk.piv;
 
@@ -72,8 +79,8 @@ __global__ void __launch_bounds__(kDecThreads) decouple_kernel(DecParams P) {
   // K_sn_r = K_sr - K_ss T     (k x r), in the L buffer for now
   cta_gemm_tiled(L, k, Ksr, n, Kss, n, false, T, k, false, k, r, k, tile);
   // X = (K_rr - T^T K_sr) - K_r_sn T
-  cta_gemm_tiled(X, r, Krr, n, T, k, true, Ksr, n, false, r, r, k, tile);
-  cta_gemm_tiled(X, r, X, r, U, r, false, T, k, false, r, r, k, tile);
+  cta_gemm_tiled(Xk, r, Krr, n, T, k, true, Ksr, n, false, r, r, k, tile);
+  cta_gemm_tiled(Xk, r, Xk, r, U, r, false, T, k, false, r, r, k, tile);
   // K is done with: stage X, K_r_sn and K_sn_r in its place (r ldx + 2 k r
   // <= n^2) and invert X there (Gauss-Jordan, partial pivoting).  X's
   // leading dimension is odd where that fits (r <= k^2): the elimination's
@@ -82,7 +89,7 @@ __global__ void __launch_bounds__(kDecThreads) decouple_kernel(DecParams P) {
   double* Xw = kbuf;
   double* Krsn = Xw + ldx * r;  // r x k
   double* Ksnr = Krsn + r * k;  // k x r
-  for (int e = threadIdx.x; e < r * r; e += kDecThreads) Xw[e % r + ldx * (e / r)] = X[e];
+  for (int e = threadIdx.x; e < r * r; e += kDecThreads) Xw[e % r + ldx * (e / r)] = Xk[e];
   for (int e = threadIdx.x; e < r * k; e += kDecThreads) {
     Krsn[e] = U[e];
     Ksnr[e] = L[e];
@@ -113,6 +120,10 @@ __global__ void __launch_bounds__(kDecThreads) decouple_kernel(DecParams P) {
   // U = X^{-1} K_r_sn,  L = K_sn_r X^{-1}
   cta_gemm_tiled(U, r, nullptr, 0, Xw, ldx, false, Krsn, r, false, r, k, r, tile, 1.0);
   cta_gemm_tiled(L, k, nullptr, 0, Ksnr, k, false, Xw, ldx, false, k, r, r, tile, 1.0);
+  if (tk.X0) {
+    cta_gemm_tiled(Ksnr, k, Ksnr, k, L, k, false, Xk, r, false, k, r, r, tile);
+    cta_gemm_tiled(L, k, L, k, Ksnr, k, false, Xw, ldx, false, k, r, r, tile, 1.0);
+  }
   // acc = update(s, s) + L K_r_sn
   cta_gemm_tiled(acc, k, nullptr, 0, L, k, false, Krsn, r, false, k, k, r, tile, 1.0);
   for (int e = threadIdx.x; e < k * k; e += kDecThreads) {
@@ -185,6 +196,9 @@ cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* s
     return e;
   if ((e = cudaMemcpyAsync(Ksnr, tk.L, sizeof(double) * r * k, cudaMemcpyDeviceToDevice, s)))
     return e;
+  if (tk.X0 && (e = cudaMemcpyAsync(tk.X0, tk.X, sizeof(double) * r * r,
+                                    cudaMemcpyDeviceToDevice, s)))
+    return e;
   if ((e = dense_lu(tk.X, r, r, tk.piv, status, s, reinterpret_cast<int*>(tk.K + nn)))) return e;
   count_launches(1);
   identity_kernel<<<(r * r + 255) / 256, 256, 0, s>>>(Y, r);
@@ -198,6 +212,12 @@ cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* s
   if ((e = launch_gemm_tiled(tk.L, k, nullptr, 0, Ksnr, k, false, tk.X, r, false, k, r, r, 1.0,
                              s)))
     return e;
+  if (tk.X0) {
+    if ((e = launch_gemm_sub(Ksnr, k, Ksnr, k, tk.L, k, false, tk.X0, r, false, k, r, r, s)))
+      return e;
+    if ((e = launch_gemm_tiled(tk.L, k, tk.L, k, Ksnr, k, false, tk.X, r, false, k, r, r, 1.0, s)))
+      return e;
+  }
   if ((e = launch_gemm_sub(tk.acc, k, nullptr, 0, tk.L, k, false, Krsn, r, false, k, k, r, s)))
     return e;
   acc_finish_kernel<<<(k * k + 255) / 256, 256, 0, s>>>(tk.acc, k, tk.perm, tk.bid, tk.bpos,

@@ -30,12 +30,13 @@ struct IdTask {
   int proxy;      // proxy rows
   int act_off;    // into IdParams::act
   int row_off;    // into IdParams::rowdofs
-  int lda;        // leading dimension of A in the workspace
+  int lda;        // streamed launches: leading dimension of A in the workspace
   int perm_off;   // into IdParams::perm (n ints)
-  long long a_off;  // A in the workspace (doubles)
+  long long a_off;  // A (streamed) or R and the spilled columns in the workspace (doubles)
   long long t_off;  // T output (doubles), capacity n*n/4 + 1
   double cx, cy, rad, pw;  // proxy circle centre, radius, weight
   int sk;         // > 0: on-chip CTA factors the sk x n row sketch S A instead of A
+  int nres;       // spilled launches: columns resident in shared memory
   int pshift;     // sketched tasks: proxy circle of kNumProxy >> pshift points
 };
 
@@ -73,30 +74,40 @@ struct IdParams {
   const double* proxy_dir;  // cos/sin table, 2 * kNumProxy doubles
   double tol;
   int m_cap, n_cap;  // streaming launches: maxima over the launch (shared-memory layout)
-  long long col_cap;  // unused by the kernels (kept for the host's bookkeeping)
   long long onchip_smem;  // on-chip launches: dynamic shared memory per CTA, the
                           // largest id_onchip_smem_bytes over the launch's tasks
 };
-// Shared memory of one on-chip CTA for an m x n box in a G-CTA cluster (the
-// layout is per task, so boxes of different sizes share a launch).
-size_t id_onchip_smem_bytes(int m, int n, int G);
-// ... and for a sketched box (sk sketch rows) in a G-CTA cluster.
-size_t id_sketch_smem_bytes(int sk, int n, int G);
 
 // launch_id group codes: G (1, 2, 4, 8) streams the matrix through HBM/L2
-// with G CTAs per box; kOnChip + G (G = 1 .. 16) keeps it in the shared
-// memory of a G-CTA cluster.
-constexpr int kOnChip = 100;
-// Column stride of an on-chip ID matrix with m rows: the smallest >= m
-// that is 4 mod 16 doubles.  The trailing update gives each column a group
-// of L lanes (L = 4 .. 32) reading consecutive rows; with the stride 4 mod
-// 16 the four 4-lane groups of a half-warp start 4 banks apart (disjoint),
-// the two 8-lane groups overlap in half their banks.  Measured on a B200
-// (deep-level IDs of the Stokes workload): the QR loop 23% faster than with
-// an odd stride, 9% faster than with 8 mod 16.
-inline int onchip_lda(int m) { return m + ((4 - m % 16) + 16) % 16; }
-// Nonzero if an on-chip launch of this size can be scheduled on the device.
-int id_cluster_fits(int group, int m_cap, int n_cap, size_t col_cap);
+// with G CTAs per box; kTile + 100 t + G keeps the matrix or its row sketch
+// (IdTask::sk rows) in the registers of a G-CTA cluster, tile shape t;
+// kOnChip + G (G = 1 .. 16) keeps the matrix in the cluster's shared memory,
+// kSketched + G (G = 8, 16) the sketch, kSpilled + G (G = 8, 16) the first
+// IdTask::nres columns, the others in the workspace.
+constexpr int kOnChip = 100, kSketched = 200, kSpilled = 300, kTile = 1000;
+// Rows of an on-chip ID matrix over a G-CTA cluster: every CTA gets the same
+// count of near rows (a zero row where they do not divide).
+__host__ __device__ inline int id_padded_rows(int n_row, int proxy, int G) {
+  return 2 * ((n_row + G - 1) / G) * G + proxy;
+}
+// Smallest register tile that holds an m x n box (m = sk rows for a sketched
+// one) in a G-CTA cluster; -1: none.
+int id_tile(int m, int n, int G);
+// Dynamic shared memory of a CTA of an on-chip launch (group >= kOnChip) for
+// such a box.
+size_t id_group_smem_bytes(int group, int m, int n, int nres);
+// Shared memory of one on-chip CTA for an m x n box (m = sk rows for a
+// sketched one) in a G-CTA cluster with nres columns resident (the layout is
+// per task, so boxes of different sizes share a launch).
+size_t id_onchip_smem_bytes(int m, int n, int G, int nres);
+// Columns of an m x n box that fit the shared memory of a G-CTA cluster (n:
+// all of them; 0: not even the bookkeeping fits).
+int id_resident_columns(int m, int n, int G);
+// Workspace of an on-chip box (doubles): R's rows and the spilled columns.
+long long id_workspace_doubles(int m, int n, int G, int nres);
+// Nonzero if a G-CTA cluster with full shared memory can be scheduled.
+int id_cluster_fits(int G);
+cudaError_t launch_id_cluster(const IdParams& p, int group, cudaStream_t s);
 
 // Launches one ID per task with a cluster of CTAs per task (group codes above).
 cudaError_t launch_id(const IdParams& p, int group, cudaStream_t s);
@@ -136,6 +147,7 @@ struct DecTask {
   double* X;             // X_rr^{-1}, r x r, ld r (written by the decoupling)
   double* acc;           // accumulated update on the skeleton, k x k
   int* piv;              // r ints of scratch (pivots of the inversion)
+  double* X0;            // r x r scratch that keeps X_rr for L's correction (null: none)
 };
 
 struct DecParams {

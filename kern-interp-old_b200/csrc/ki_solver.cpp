@@ -147,17 +147,42 @@ int pick_stream_group(long long m, long long n) {
   return 1;
 }
 
-// Smallest cluster whose shared memory holds the whole m x n matrix (group
-// code kOnChip + G), else a streaming launch.  onchip_ok[G] says whether a
-// G-CTA cluster with full shared memory can be scheduled on this device.
-int pick_group(int m, int n, const bool* onchip_ok) {
-  const long long lda = onchip_lda(m);
-  for (int G = 1; G <= 16; G *= 2) {
-    if (!onchip_ok[G]) continue;
-    const long long cols = (n + G - 1) / G * lda;
-    if (id_smem_bytes(m, n) + sizeof(double) * cols <= 227 * 1024) return kOnChip + G;
+// Launch of an exact ID (group codes of launch_id): the smallest cluster
+// whose registers hold the whole matrix; *g_slab, *nres: without registers,
+// the smallest cluster whose shared memory does, else the widest one with
+// the columns that do not fit spilled to the workspace (nres resident), else
+// a streaming launch.  onchip_ok[G] says whether a G-CTA cluster with full
+// shared memory can be scheduled on this device.
+int pick_group(int n_row, int proxy, int n, const bool* onchip_ok, int* g_slab, int* nres) {
+  auto m = [&](int G) { return id_padded_rows(n_row, proxy, G); };
+  *nres = n;
+  *g_slab = 0;
+  for (int G = 1; G <= 16 && !*g_slab; G *= 2)
+    if (onchip_ok[G] && id_resident_columns(m(G), n, G) >= n) *g_slab = kOnChip + G;
+  for (int G = 16; G >= 8 && !*g_slab; G /= 2) {
+    const int c = onchip_ok[G] ? id_resident_columns(m(G), n, G) : 0;
+    if (c > 0) {
+      *nres = c;
+      *g_slab = kSpilled + G;
+    }
   }
-  return pick_stream_group(m, n);
+  if (!*g_slab) *g_slab = pick_stream_group(2 * n_row + proxy, n);
+  for (int G = 1; G <= 16; G *= 2) {
+    const int t = onchip_ok[G] ? id_tile(m(G), n, G) : -1;
+    if (t >= 0) return kTile + 100 * t + G;
+  }
+  return *g_slab;
+}
+
+// The same for an l x n sketch; 0: none.
+int pick_sketch_group(int l, int n, const bool* onchip_ok) {
+  for (int G = 1; G <= 16; G *= 2) {
+    const int t = onchip_ok[G] ? id_tile(l, n, G) : -1;
+    if (t >= 0) return kTile + 100 * t + G;
+  }
+  for (int G = 8; G <= 16; G *= 2)
+    if (onchip_ok[G] && id_resident_columns(l, n, G) >= n) return kSketched + G;
+  return 0;
 }
 
 }  // namespace
@@ -202,6 +227,7 @@ namespace {
 // small factorization's level loop).
 struct AuxSet {
   int dev = -1;
+  bool high = false;  // the decoupling's streams have the highest priority
   cudaStream_t d = nullptr;
   cudaEvent_t ev_id[2] = {}, ev_dec = nullptr, fork = nullptr;
   cudaStream_t id[3] = {};
@@ -252,6 +278,7 @@ Solver::~Solver() {
     static_assert(kIdStreams == 3 && kDecStreams == 3, "AuxSet holds three of each");
     AuxSet a;
     cudaGetDevice(&a.dev);
+    a.high = opt_.sketch_id;
     a.d = dstream_;
     a.ev_id[0] = ev_id_[0];
     a.ev_id[1] = ev_id_[1];
@@ -440,7 +467,7 @@ int Solver::begin_factor(cudaEvent_t* ev0) {
       std::lock_guard<std::mutex> lk(g_aux_mu);
       auto& fl = aux_free();
       for (size_t i = 0; i < fl.size(); i++)
-        if (fl[i].dev == dev) {
+        if (fl[i].dev == dev && fl[i].high == opt_.sketch_id) {
           const AuxSet a = fl[i];
           fl.erase(fl.begin() + static_cast<long>(i));
           dstream_ = a.d;
@@ -466,7 +493,13 @@ int Solver::begin_factor(cudaEvent_t* ev0) {
         }
     }
     if (!dstream_) {
-      KI_CUDA(cudaStreamCreateWithFlags(&dstream_, cudaStreamNonBlocking));
+      // A preconditioner's factorization waits for its chain of
+      // decouplings (its sketched IDs finish early), a reference one for its
+      // IDs: the decouplings' blocks go first only in the former.
+      int lowest = 0, highest = 0;
+      KI_CUDA(cudaDeviceGetStreamPriorityRange(&lowest, &highest));
+      const int prio = opt_.sketch_id ? highest : lowest;
+      KI_CUDA(cudaStreamCreateWithPriority(&dstream_, cudaStreamNonBlocking, prio));
       KI_CUDA(cudaEventCreateWithFlags(&ev_id_[0], cudaEventDisableTiming));
       KI_CUDA(cudaEventCreateWithFlags(&ev_id_[1], cudaEventDisableTiming));
       KI_CUDA(cudaEventCreateWithFlags(&ev_dec_, cudaEventDisableTiming));
@@ -477,7 +510,7 @@ int Solver::begin_factor(cudaEvent_t* ev0) {
       }
       KI_CUDA(cudaEventCreateWithFlags(&dl_fork_, cudaEventDisableTiming));
       for (int i = 0; i < kDecStreams; i++) {
-        KI_CUDA(cudaStreamCreateWithFlags(&dl_streams_[i], cudaStreamNonBlocking));
+        KI_CUDA(cudaStreamCreateWithPriority(&dl_streams_[i], cudaStreamNonBlocking, prio));
         KI_CUDA(cudaEventCreateWithFlags(&dl_join_[i], cudaEventDisableTiming));
       }
       KI_CUDA(cudaStreamCreateWithFlags(&bstream_, cudaStreamNonBlocking));
@@ -499,8 +532,7 @@ int Solver::begin_factor(cudaEvent_t* ev0) {
     if (it == known.end()) {
       std::array<bool, 17> ok{};
       for (int G = 1; G <= 16; G *= 2)
-        ok[G] = id_cluster_fits(kOnChip + G, 4096, 256,
-                                (227 * 1024 - id_smem_bytes(4096, 256)) / 8) != 0;
+        ok[G] = id_cluster_fits(G) != 0;
       it = known.emplace(dev, ok).first;
     }
     for (int G = 0; G <= 16; G++) onchip_ok_[G] = it->second[G];
@@ -683,11 +715,15 @@ int Solver::finish_factor(cudaEvent_t ev0) {
     for (int level = L - 1; level > 0 && !rc; level--) {
       auto next = std::make_unique<PendingLevel>();
       const bool more = level > 1 && !(level == 2 && level1_stays());
-      if (more) {
+      // what the factorization waits for goes first: the decouplings of a
+      // preconditioner (measured on a B200: see the stream priorities), the
+      // IDs of a reference factorization
+      if (opt_.sketch_id) rc = decouple_level(cur.get());
+      if (!rc && more) {
         rc = id_launch(level - 1, next.get());
         refreshed = level - 1;
       }
-      if (!rc) rc = decouple_level(cur.get());
+      if (!rc && !opt_.sketch_id) rc = decouple_level(cur.get());
       if (!rc && more) rc = id_finish(next.get());
       if (!more) break;
       cur = std::move(next);
@@ -807,26 +843,8 @@ int Solver::id_launch(int level, PendingLevel* pl) {
         c.m = 2 * c.I + P;
       }
       if (c.m == 0) continue;
-      c.g = pick_group(c.m, c.n, onchip_ok_);
+      c.g = pick_group(c.I, c.m - 2 * c.I, c.n, onchip_ok_, &c.g_slab, &c.nres);
       if (opt_.sketch_id) {
-        // A level whose boxes, each spread over the widest cluster that
-        // still leaves a CTA 12 columns, fit one wave at two CTAs per SM
-        // takes that width: the pivoted QR's steps shrink with the columns
-        // a CTA owns (measured on a B200, the Stokes workload's level-2
-        // IDs: 0.96 -> 0.72 ms).  Otherwise the smallest cluster whose
-        // CTAs' shares of the sketch leave room for two CTAs per SM (a
-        // single CTA per SM leaves the SM idle at every barrier of the
-        // pivoted QR), else the smallest that fits.
-        auto fit = [&](int l) {  // cluster size for an l-row sketch, 0: none
-          for (int G = 16; G >= 2; G /= 2)
-            if (onchip_ok_[G] && c.n >= 12 * G && nids * G <= 2 * num_sms_ &&
-                id_sketch_smem_bytes(l, c.n, G) <= size_t{113} * 1024)
-              return G;
-          for (const size_t cap : {size_t{113} * 1024, size_t{227} * 1024})
-            for (int G = 1; G <= 16; G *= 2)
-              if (onchip_ok_[G] && id_sketch_smem_bytes(l, c.n, G) <= cap) return G;
-          return 0;
-        };
         // the full sketch (n + 16 rows) must be possible; on a level of many
         // boxes the box is then sketched with rows sized by the level below's
         // ranks, and decomposed again with the full sketch if those do not
@@ -835,13 +853,16 @@ int Solver::id_launch(int level, PendingLevel* pl) {
         // whole launch and rank read-back on the factorization's critical
         // path)
         const int l = sketch_rows(c.n);
-        const int G_full = c.m > l + 64 && l >= 32 ? fit(l) : 0;  // (bucket runs need l >= 32)
-        if (G_full) {
+        const int g_full =
+            c.m > l + 64 && l >= 32 ? pick_sketch_group(l, c.n, onchip_ok_) : 0;
+        if (g_full) {
           const int ls = nids > kShortSketchMinBoxes ? sketch_rows_hint(c.n, rank_hint_) : l;
-          const int G_short = ls < l ? fit(ls) : 0;
-          c.sk = G_short ? ls : l;
-          c.g = kOnChip + (G_short ? G_short : G_full);
-          c.g_full = G_short ? kOnChip + G_full : 0;
+          const int g_short = ls < l ? pick_sketch_group(ls, c.n, onchip_ok_) : 0;
+          c.sk = g_short ? ls : l;
+          c.g = g_short ? g_short : g_full;
+          c.g_full = g_short ? g_full : 0;
+          c.g_slab = 0;
+          c.nres = c.n;
         }
         if (c.sk && level > 2) c.m = 2 * c.I + (P >> opt_.proxy_shift);
       }
@@ -853,6 +874,15 @@ int Solver::id_launch(int level, PendingLevel* pl) {
   for (int q = 0; q < nids; q++)
     if (keep[q]) cand.push_back(std::move(all[q]));
   if (cand.empty()) return 0;
+  // A box in registers takes more CTAs than one in shared memory (160 KB of
+  // an SM's registers hold matrix entries, 220 KB of its shared memory) but
+  // is done sooner, so a level that fits the GPU in registers takes them and
+  // a fuller one the smaller clusters.
+  int ctas = 0;
+  for (const Cand& c : cand) ctas += c.g % 100;
+  if (ctas > num_sms_)
+    for (Cand& c : cand)
+      if (c.g_slab && c.g >= kTile && c.g_slab % 100 < c.g % 100) c.g = c.g_slab;
   // grouped by cluster size, the group holding the widest ID matrix first
   // (its launch then takes SMs before the many-box launch fills them: the
   // few big boxes are each level's longest tasks), and inside a group the
@@ -881,7 +911,8 @@ int Solver::id_launch(int level, PendingLevel* pl) {
   for (int q = 0; q < nc; q++) {  // offsets
     const Cand& c = cand[q];
     IdTask& t = tasks[q];
-    t.lda = c.sk ? onchip_lda(c.sk) : c.g >= kOnChip ? onchip_lda(c.m) : (c.m + 3) & ~3;
+    t.lda = (c.m + 3) & ~3;
+    t.nres = c.nres;
     t.act_off = static_cast<int>(act_total);
     t.row_off = static_cast<int>(rows_total);
     t.perm_off = perm_total;
@@ -889,7 +920,13 @@ int Solver::id_launch(int level, PendingLevel* pl) {
     t.t_off = t_total;
     act_total += c.n;
     rows_total += c.rows.size();
-    if (c.g < kOnChip) a_total += static_cast<long long>(t.lda) * c.n;  // on-chip: none
+    if (c.g < kOnChip) {
+      a_total += static_cast<long long>(t.lda) * c.n;
+    } else {  // (a sketched box decomposed again may take a wider cluster)
+      const int G = std::max(c.g % 100, c.g_full % 100);
+      a_total += id_workspace_doubles(c.sk ? c.n : id_padded_rows(c.I, c.m - 2 * c.I, G), c.n, G,
+                                      c.nres);
+    }
     t_total += static_cast<long long>(c.n) * c.n / 4 + 1;
     perm_total += c.n;
   }
@@ -955,14 +992,17 @@ int Solver::id_launch(int level, PendingLevel* pl) {
     int m_cap = 0, n_cap = 0;
     long long onchip = 0;
     const int g0 = cand[q0].g;
-    const int G = g0 >= kOnChip ? g0 - kOnChip : 0;
+    const int G = g0 >= kOnChip ? g0 % 100 : 0;
     while (q1 < nc && cand[q1].g == g0) {
       const int mm = std::max(m_cap, cand[q1].m), nn = std::max(n_cap, cand[q1].n);
       if (G) {
         // per-task layout: the launch needs the largest single task's share
         onchip = std::max<long long>(
-            onchip, cand[q1].sk ? id_sketch_smem_bytes(cand[q1].sk, cand[q1].n, G)
-                                : id_onchip_smem_bytes(cand[q1].m, cand[q1].n, G));
+            onchip, id_group_smem_bytes(g0,
+                                        cand[q1].sk ? cand[q1].sk
+                                                    : id_padded_rows(cand[q1].I,
+                                                                     cand[q1].m - 2 * cand[q1].I, G),
+                                        cand[q1].n, cand[q1].nres));
       } else if (q1 > q0 && id_smem_bytes(mm, nn) > 227 * 1024) {
         break;
       }
@@ -1042,7 +1082,6 @@ int Solver::id_rerun_full(PendingLevel* pl) {
     if (!c.g_full) return fail("interpolative decomposition: sketch too short for a box");
     t2[u] = pl->tasks[qs[u]];
     t2[u].sk = sketch_rows(c.n);
-    t2[u].lda = onchip_lda(t2[u].sk);
     c.sk = t2[u].sk;
     c.g = c.g_full;
   }
@@ -1058,7 +1097,7 @@ int Solver::id_rerun_full(PendingLevel* pl) {
     int n_cap = 0;
     while (q1 < qs.size() && pl->cand[qs[q1]].g == g) {
       const IdCand& c = pl->cand[qs[q1]];
-      smem = std::max<long long>(smem, id_sketch_smem_bytes(c.sk, c.n, g - kOnChip));
+      smem = std::max<long long>(smem, id_group_smem_bytes(g, c.sk, c.n, c.n));
       n_cap = std::max(n_cap, c.n);
       q1++;
     }
@@ -1142,6 +1181,7 @@ int Solver::id_finish(PendingLevel* pl) {
         const double sd = sd_;  // dofs per node record
         double bytes = 4.0 * (c.I + 2 * n) + 64.0 * (c.I + c.n) / sd + 8.0 * k * (n - k);
         if (c.g < kOnChip) bytes += 16.0 * c.m * n;
+        if (c.nres < c.n) bytes += 16.0 * c.m * (n - c.nres);
         qr_v[q] = qr;
         bytes_v[q] = bytes;
         if (k == 0) continue;
@@ -1230,7 +1270,7 @@ int Solver::decouple_boxes(PendingLevel* pl) {
   });
   std::vector<long long> bid_off(ncomp + 1, 0), tab_off(ncomp + 1, 0);
   long long scratch_total = 0;
-  std::vector<long long> k_off(ncomp);
+  std::vector<long long> k_off(ncomp), x0_off(ncomp);
   int n_max = 0;
   size_t fac_total = 0, piv_total = 0;
   for (int t = 0; t < ncomp; t++) {
@@ -1246,6 +1286,8 @@ int Solver::decouple_boxes(PendingLevel* pl) {
     } else {
       n_max = std::max(n_max, n);
     }
+    x0_off[t] = scratch_total;
+    if (!opt_.sketch_id) scratch_total += static_cast<long long>(r) * r;
     fac_total += static_cast<size_t>(k) * r * 2 + static_cast<size_t>(r) * r +
                  static_cast<size_t>(k) * k;
     piv_total += r;
@@ -1254,6 +1296,7 @@ int Solver::decouple_boxes(PendingLevel* pl) {
       // K_BN entries (~20 flops each), T^T K_ss, T^T K_sr, K_r_sn T, K_ss T,
       // X_rr^-1 (Gauss-Jordan), U = X^-1 K_r_sn, L = K_sn_r X^-1, L K_r_sn
       dec_flops += 20.0 * dn * dn + 2.0 * dr * dr * dr + 8.0 * dr * dr * dk + 6.0 * dr * dk * dk;
+      if (!opt_.sketch_id) dec_flops += 4.0 * dr * dr * dk;  // L's correction
       solve_bytes += 8.0 * (4.0 * dk * dr + dr * dr);
     }
   }
@@ -1319,6 +1362,7 @@ int Solver::decouple_boxes(PendingLevel* pl) {
     d.X = bd.X;
     d.acc = bd.acc;
     d.piv = bd.piv;
+    d.X0 = opt_.sketch_id ? nullptr : scr + x0_off[t];
   }
   // small boxes first in one batched launch, then each large box
   std::vector<DecTask> small, large;

@@ -282,6 +282,8 @@ class Solver {
   struct IdCand {
     int box = -1, n = 0, m = 0, I = 0, g = 0, sk = 0;
     int g_full = 0;  // sketched with fewer than n + 16 rows: the cluster for n + 16
+    int g_slab = 0;  // launch group without register tiles (exact boxes)
+    int nres = 0;    // columns resident in shared memory (kSpilled launches)
     std::vector<int> rows;
   };
   struct PendingLevel {
