@@ -39,97 +39,314 @@ __device__ __forceinline__ double upd_lookup(const int* bid, const int* bpos,
   return blk.acc[bpos[a] + static_cast<long long>(blk.size) * bpos[b]];
 }
 
-// Boxes with n <= kSmemN keep K_BN, and then X_rr, in shared memory.
-constexpr int kSmemN = kDecoupleSmemN;
+// Leading dimension of a matrix in shared memory whose DMMA fragments are
+// read in place: 4 mod 8 doubles, so the four inner indices (or rows) of a
+// half-warp's fragment, a stride apart, start 4 or 12 banks of 16 apart and
+// its four consecutive entries fill the gaps: no two lanes share a bank.
+__host__ __device__ inline int frag_ld(int n) { return n + ((4 - n % 8) + 8) % 8; }
 
-__global__ void __launch_bounds__(kDecThreads) decouple_kernel(DecParams P) {
+// The CTA's product op(A) op(B) (m x n, inner kk) on the FP64 tensor cores,
+// both operands in shared memory with a frag_ld stride; out(i, j, v)
+// receives every entry.  A warp computes 16 x 16 blocks (2 x 2 DMMA blocks)
+// straight from the operands: no staging, no barriers.
+template <bool TA, bool TB, class Out>
+__device__ __forceinline__ void cta_mma(const double* A, int lda, const double* B, int ldb, int m,
+                                        int n, int kk, Out out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int fr = lane >> 2, fk = lane & 3;
+  const int tm = (m + 15) / 16, tn = (n + 15) / 16;
+  for (int t = warp; t < tm * tn; t += kDecThreads / 32) {
+    const int i0 = t % tm * 16, j0 = t / tm * 16;
+    // (rows and columns past the edge repeat the last: never stored)
+    const double *pa[2], *pb[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int i = min(i0 + 8 * h + fr, m - 1), j = min(j0 + 8 * h + fr, n - 1);
+      pa[h] = TA ? A + static_cast<size_t>(lda) * i : A + i;
+      pb[h] = TB ? B + j : B + static_cast<size_t>(ldb) * j;
+    }
+    double acc[2][2][2] = {};
+#pragma unroll 4
+    for (int l0 = 0; l0 < kk; l0 += 4) {
+      const int l = l0 + fk;
+      double fa[2], fb[2];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        fa[h] = l < kk ? pa[h][TA ? l : lda * l] : 0.0;
+        fb[h] = l < kk ? pb[h][TB ? ldb * l : l] : 0.0;
+      }
+#pragma unroll
+      for (int x = 0; x < 2; x++)
+#pragma unroll
+        for (int y = 0; y < 2; y++) dmma_8x8x4(acc[x][y][0], acc[x][y][1], fa[x], fb[y]);
+    }
+#pragma unroll
+    for (int x = 0; x < 2; x++)
+#pragma unroll
+      for (int y = 0; y < 2; y++)
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+          const int i = i0 + 8 * x + fr, j = j0 + 8 * y + 2 * fk + v;
+          if (i < m && j < n) out(i, j, acc[x][y][v]);
+        }
+  }
+}
+
+// Gauss-Jordan inversion of the r x r matrix X (shared memory, stride ld) by
+// the CTA's 8 warps with the matrix in registers: warp w owns the columns
+// c % 8 == w, its lanes the rows (lane + 32 s in slot s), a thread CW x RS
+// entries.  Partial pivoting, rows never exchanged: step j eliminates column
+// j with row p_j (the largest |x(i, j)| among the rows not yet pivots, the
+// first on ties; a NaN counts as 0).  The owner warp of column j finds p_j
+// and publishes the column (double-buffered by step parity), one barrier, and
+// every warp updates its columns: row p_j's entries come by shuffle from the
+// lane that holds them.  In place the result B holds X^{-1}(j, q) =
+// B(p_j, p^{-1}(q)); it is stored to X in X^{-1}'s own order.  pr, pi: p and
+// p^{-1}.  Returns nonzero when a pivot was 0, infinite or NaN.
+// A step moves the pivot column through shared memory once; with the matrix
+// there (a thread per row segment) it moved 24 bytes per entry and step:
+// 6,000 against 900 cycles a step for r = 70 with the SM shared.
+template <int CW, int RS>
+__device__ __forceinline__ int cta_gj_regs(double* X, int ld, int r, double* colj, int* sp, int* pr,
+                                           int* pi) {
+  constexpr int RP = 32 * RS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double x[CW][RS];
+#pragma unroll
+  for (int u = 0; u < CW; u++) {
+    const int c = u * 8 + warp;
+#pragma unroll
+    for (int s = 0; s < RS; s++) {
+      const int i = lane + 32 * s;
+      x[u][s] = c < r && i < r ? X[i + static_cast<size_t>(ld) * c] : 0.0;
+    }
+  }
+  unsigned used = 0;  // slots whose row has been a pivot
+  int info = 0;
+  for (int j = 0; j < r; j++) {
+    double* cj = colj + (j & 1) * RP;
+    if ((j & 7) == warp) {
+      // (comparing columns, not u: see cta_mma's callers' register arrays,
+      // which an equality on the index would turn into local memory)
+      double y[RS];
+#pragma unroll
+      for (int u = 0; u < CW; u++)
+        if (u * 8 + warp == j) {
+#pragma unroll
+          for (int s = 0; s < RS; s++) y[s] = x[u][s];
+        }
+      unsigned long long key = 0;
+      int idx = 0x7fffffff;
+#pragma unroll
+      for (int s = 0; s < RS; s++) {
+        const int i = lane + 32 * s;
+        double v = fabs(y[s]);
+        if (v != v) v = 0.0;
+        const unsigned long long k = static_cast<unsigned long long>(__double_as_longlong(v));
+        if (i < r && !(used >> s & 1) && (idx == 0x7fffffff || k > key)) {
+          key = k;
+          idx = i;
+        }
+        cj[i] = y[s];
+      }
+      unsigned long long gk;
+      int p;
+      warp_argmax_bits(key, idx, &gk, &p);
+      if (lane == 0) {
+        sp[j & 1] = p;
+        pr[j] = p;
+        pi[p] = j;
+      }
+    }
+    __syncthreads();
+    const int p = sp[j & 1];
+    const double piv = cj[p];
+    if (!(fabs(piv) > 0.0) || isinf(piv)) info = 1;  // (0, NaN or infinite)
+    const double inv = 1.0 / piv;
+    double f[RS];
+#pragma unroll
+    for (int s = 0; s < RS; s++) f[s] = lane + 32 * s == p ? 0.0 : cj[lane + 32 * s];
+#pragma unroll
+    for (int s = 0; s < RS; s++) {
+      const int t = p - 32 * s;
+      if (static_cast<unsigned>(t) < 32u) {  // the slot of row p
+#pragma unroll
+        for (int u = 0; u < CW; u++) {
+          const double q = __shfl_sync(0xffffffffu, x[u][s], t) * inv;
+#pragma unroll
+          for (int h = 0; h < RS; h++) x[u][h] = fma(-f[h], q, x[u][h]);
+          if (lane == t) x[u][s] = q;
+        }
+        if (lane == t) used |= 1u << s;
+      }
+    }
+    if ((j & 7) == warp) {
+#pragma unroll
+      for (int u = 0; u < CW; u++)
+        if (u * 8 + warp == j) {
+#pragma unroll
+          for (int s = 0; s < RS; s++) x[u][s] = lane + 32 * s == p ? inv : -f[s] * inv;
+        }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < CW; u++) {
+    const int c = u * 8 + warp;
+    if (c < r) {
+      double* col = X + static_cast<size_t>(ld) * pr[c];
+#pragma unroll
+      for (int s = 0; s < RS; s++) {
+        const int i = lane + 32 * s;
+        if (i < r) col[pi[i]] = x[u][s];
+      }
+    }
+  }
+  __syncthreads();
+  return info;
+}
+
+// Shared memory of a box: K_BN (in place K_r_sn, K_sn_r, X_rr and its
+// inverse), T and later L, the pivot column twice, pivots, per-dof ints; with
+// L's correction the staging tile of a product with an operand in global
+// memory.
+struct DecLayout {
+  int ldn, ldk;
+  size_t tl, tile, colj, ints, bytes;  // offsets in doubles, total bytes
+};
+__host__ __device__ inline DecLayout dec_layout(int n, int k, bool correct) {
+  DecLayout d;
+  const int r = n - k;
+  d.ldn = frag_ld(n);
+  d.ldk = frag_ld(k);
+  d.tl = static_cast<size_t>(n) * d.ldn;
+  const size_t t = static_cast<size_t>(d.ldk) * r, nodes = 8 * static_cast<size_t>(n);
+  d.tile = d.tl + (((t > nodes ? t : nodes) + 1) & ~static_cast<size_t>(1));
+  d.colj = d.tile + (correct ? kGemmTileDoubles : 0);
+  d.ints = d.colj + 2 * 160;
+  d.bytes = sizeof(double) * d.ints + sizeof(int) * (5 * static_cast<size_t>(n) + 4);
+  return d;
+}
+
+// FAST: entries by contracted arithmetic (a preconditioner's, whose sketched
+// IDs use it too); else the reference's bits, and L corrected.
+template <int CW, int RS, int MINB, bool FAST>
+__global__ void __launch_bounds__(kDecThreads, MINB) decouple_kernel(DecParams P) {
   extern __shared__ __align__(16) double dsm[];
-  double* tile = dsm;                     // kGemmTileDoubles
-  double* red = tile + kGemmTileDoubles;  // 64
-  double* kbuf = red + 64;                // n*n when staged
   const DecTask tk = P.tasks[blockIdx.x];
-  const int n = tk.n, k = tk.k, r = n - k;  // n <= kSmemN: the host sends larger boxes
-  const int* act = tk.act;                  // through decouple_large
-  const int* perm = tk.perm;
-  const int* bid = tk.bid;
-  const int* bpos = tk.bpos;
-  const double* T = tk.T;
-  double* K = kbuf;
-  double* L = tk.L;
-  double* U = tk.U;
-  double* X = tk.X;
-  double* Xk = tk.X0 ? tk.X0 : X;  // X_rr itself, kept where L is corrected
-  double* acc = tk.acc;
-  int* piv = tk.piv;
+  const int n = tk.n, k = tk.k, r = n - k;
+  const DecLayout lay = dec_layout(n, k, !FAST);
+  const int ldn = lay.ldn, ldk = lay.ldk;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* K = dsm;
+  double* TL = dsm + lay.tl;
+  double* colj = dsm + lay.colj;
+  int* prow = reinterpret_cast<int*>(dsm + lay.ints);  // n
+  int* pinv = prow + n;                                 // n
+  int* dof = pinv + n;                                  // n, pivot order; likewise:
+  int* sbid = dof + n;                                  // n
+  int* sbpos = sbid + n;                                // n
+  int* sp = sbpos + n;                                  // 2
 
-  // K_BN in pivot order
-  for (int e = threadIdx.x; e < n * n; e += kDecThreads) {
-    const int a = e % n, b = e / n;
-    const int pa = perm[a], pb = perm[b];
-    const double kv = boundary_entry(P.pde, P.nodes, act[pa], act[pb]);
-    K[e] = kv - upd_lookup(bid, bpos, tk.blocks, pa, pb);
+  // ---- K_BN in pivot order: a lane keeps its row's node record and block,
+  // the columns' records pass by broadcast, four at a time (their update
+  // entries are loads from global memory)
+  Node* nd = reinterpret_cast<Node*>(TL);
+  const int sh = P.pde == kStokes ? 1 : 0;
+  for (int a = threadIdx.x; a < n; a += kDecThreads) {
+    const int pa = tk.perm[a], d = tk.act[pa];
+    dof[a] = d;
+    nd[a] = P.nodes[d >> sh];
+    sbid[a] = tk.bid[pa];
+    sbpos[a] = tk.bpos[pa];
   }
   __syncthreads();
-  const double* Kss = K;
-  const double* Krs_in = K + k;
-  const double* Ksr = K + static_cast<long long>(n) * k;
-  const double* Krr = K + k + static_cast<long long>(n) * k;
-  // K_r_sn = K_rs - T^T K_ss   (r x k), in the U buffer for now
-  cta_gemm_tiled(U, r, Krs_in, n, T, k, true, Kss, n, false, r, k, k, tile);
-  // K_sn_r = K_sr - K_ss T     (k x r), in the L buffer for now
-  cta_gemm_tiled(L, k, Ksr, n, Kss, n, false, T, k, false, k, r, k, tile);
-  // X = (K_rr - T^T K_sr) - K_r_sn T
-  cta_gemm_tiled(Xk, r, Krr, n, T, k, true, Ksr, n, false, r, r, k, tile);
-  cta_gemm_tiled(Xk, r, Xk, r, U, r, false, T, k, false, r, r, k, tile);
-  // K is done with: stage X, K_r_sn and K_sn_r in its place (r ldx + 2 k r
-  // <= n^2) and invert X there (Gauss-Jordan, partial pivoting).  X's
-  // leading dimension is odd where that fits (r <= k^2): the elimination's
-  // row operations, a thread per column, then hit distinct banks
-  const int ldx = (r | 1) * r + 2 * k * r <= n * n ? (r | 1) : r;
-  double* Xw = kbuf;
-  double* Krsn = Xw + ldx * r;  // r x k
-  double* Ksnr = Krsn + r * k;  // k x r
-  for (int e = threadIdx.x; e < r * r; e += kDecThreads) Xw[e % r + ldx * (e / r)] = Xk[e];
-  for (int e = threadIdx.x; e < r * k; e += kDecThreads) {
-    Krsn[e] = U[e];
-    Ksnr[e] = L[e];
+  {
+    const int rb = (n + 31) / 32, nch = (8 + rb - 1) / rb;
+    for (int w = warp; w < rb * nch; w += kDecThreads / 32) {
+      const int a = 32 * (w % rb) + lane, ch = w / rb;
+      const bool in = a < n;
+      const int aa = in ? a : n - 1;
+      const Node na = nd[aa];
+      const int da = dof[aa], ba = sbid[aa], pa = sbpos[aa];
+      const double* acc = ba >= 0 ? tk.blocks[ba].acc + pa : nullptr;
+      const int size = ba >= 0 ? tk.blocks[ba].size : 0;
+      const int b1 = (ch + 1) * n / nch;
+      for (int b0 = ch * n / nch; b0 < b1; b0 += 4) {
+        double up[4], v[4];
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+          const int b = min(b0 + h, b1 - 1);
+          up[h] = ba >= 0 && sbid[b] == ba ? acc[static_cast<size_t>(size) * sbpos[b]] : 0.0;
+        }
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+          const int b = min(b0 + h, b1 - 1);
+          v[h] = pair_entry<FAST>(P.pde, na, da, nd[b], dof[b]) - up[h];
+        }
+#pragma unroll
+        for (int h = 0; h < 4; h++)
+          if (in && b0 + h < b1) K[a + static_cast<size_t>(ldn) * (b0 + h)] = v[h];
+      }
+    }
   }
   __syncthreads();
-  // Gauss-Jordan with the pivot rows left in place (one barrier per step);
-  // the result B gives X^{-1}(j, q) = B(p_j, p^{-1}(q)), gathered into X
-  // in global memory and read back into shared memory for the products
-  int* prow = reinterpret_cast<int*>(tile);  // the tile is free until U, L
-  int* pinv = prow + kSmemN;
-  unsigned long long* slot_key = reinterpret_cast<unsigned long long*>(pinv + kSmemN);
-  int* slot_row = reinterpret_cast<int*>(slot_key + 64);
-  double* colj = reinterpret_cast<double*>(slot_row + 64);  // 2 r
-  const int info = cta_gj_invert_inplace(Xw, r, ldx, prow, slot_key, slot_row, colj);
+  for (int c = warp; c < r; c += kDecThreads / 32)
+    for (int l = lane; l < k; l += 32)
+      TL[l + static_cast<size_t>(ldk) * c] = tk.T[l + static_cast<size_t>(k) * c];
+  __syncthreads();
+  double* Kss = K;
+  double* Krs = K + k;
+  double* Ksr = K + static_cast<size_t>(ldn) * k;
+  double* Krr = Ksr + k;
+  auto minus = [&](double* C) {
+    return [C, ldn](int i, int j, double v) { C[i + static_cast<size_t>(ldn) * j] -= v; };
+  };
+  // K_r_sn = K_rs - T^T K_ss,  X = (K_rr - T^T K_sr) - K_r_sn T,  K_sn_r =
+  // K_sr - K_ss T, each in place (an entry is read as C only by the thread
+  // that replaces it)
+  cta_mma<true, false>(TL, ldk, Kss, ldn, r, k, k, minus(Krs));
+  cta_mma<true, false>(TL, ldk, Ksr, ldn, r, r, k, minus(Krr));
+  __syncthreads();
+  cta_mma<false, false>(Krs, ldn, TL, ldk, r, r, k, minus(Krr));
+  cta_mma<false, false>(Kss, ldn, TL, ldk, k, r, k, minus(Ksr));
+  __syncthreads();
+  if (!FAST)  // X_rr itself, for L's correction
+    for (int c = warp; c < r; c += kDecThreads / 32)
+      for (int i = lane; i < r; i += 32)
+        tk.X0[i + static_cast<size_t>(r) * c] = Krr[i + static_cast<size_t>(ldn) * c];
+  const int info = cta_gj_regs<CW, RS>(Krr, ldn, r, colj, sp, prow, pinv);
   if (info && threadIdx.x == 0) atomicExch(P.status, 1);
-  for (int j = threadIdx.x; j < r; j += kDecThreads) {
-    pinv[prow[j]] = j;
-    piv[j] = prow[j];
-  }
+  for (int j = threadIdx.x; j < r; j += kDecThreads) tk.piv[j] = prow[j];
+  for (int c = warp; c < r; c += kDecThreads / 32)
+    for (int i = lane; i < r; i += 32)
+      tk.X[i + static_cast<size_t>(r) * c] = Krr[i + static_cast<size_t>(ldn) * c];
+  // U = X^{-1} K_r_sn,  L = K_sn_r X^{-1}  (in T's place)
+  cta_mma<false, false>(Krr, ldn, Krs, ldn, r, k, r, [&](int i, int j, double v) {
+    tk.U[i + static_cast<size_t>(r) * j] = v;
+  });
+  cta_mma<false, false>(Ksr, ldn, Krr, ldn, k, r, r, [&](int i, int j, double v) {
+    TL[i + static_cast<size_t>(ldk) * j] = v;
+  });
   __syncthreads();
-  for (int e = threadIdx.x; e < r * r; e += kDecThreads) {
-    const int j = e % r, q = e / r;
-    X[e] = Xw[prow[j] + ldx * pinv[q]];
+  if (!FAST) {
+    cta_gemm_tiled(Ksr, ldn, Ksr, ldn, TL, ldk, false, tk.X0, r, false, k, r, r, dsm + lay.tile);
+    cta_mma<false, false>(Ksr, ldn, Krr, ldn, k, r, r, [&](int i, int j, double v) {
+      TL[i + static_cast<size_t>(ldk) * j] += v;
+    });
+    __syncthreads();
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < r * r; e += kDecThreads) Xw[e % r + ldx * (e / r)] = X[e];
-  __syncthreads();
-  // U = X^{-1} K_r_sn,  L = K_sn_r X^{-1}
-  cta_gemm_tiled(U, r, nullptr, 0, Xw, ldx, false, Krsn, r, false, r, k, r, tile, 1.0);
-  cta_gemm_tiled(L, k, nullptr, 0, Ksnr, k, false, Xw, ldx, false, k, r, r, tile, 1.0);
-  if (tk.X0) {
-    cta_gemm_tiled(Ksnr, k, Ksnr, k, L, k, false, Xk, r, false, k, r, r, tile);
-    cta_gemm_tiled(L, k, L, k, Ksnr, k, false, Xw, ldx, false, k, r, r, tile, 1.0);
-  }
+  for (int c = warp; c < r; c += kDecThreads / 32)
+    for (int l = lane; l < k; l += 32)
+      tk.L[l + static_cast<size_t>(k) * c] = TL[l + static_cast<size_t>(ldk) * c];
   // acc = update(s, s) + L K_r_sn
-  cta_gemm_tiled(acc, k, nullptr, 0, L, k, false, Krsn, r, false, k, k, r, tile, 1.0);
-  for (int e = threadIdx.x; e < k * k; e += kDecThreads) {
-    const int i = e % k, j = e / k;
-    acc[e] += upd_lookup(bid, bpos, tk.blocks, perm[i], perm[j]);
-  }
+  cta_mma<false, false>(TL, ldk, Krs, ldn, k, k, r, [&](int i, int j, double v) {
+    const int bi = sbid[i];
+    double up = 0.0;
+    if (bi >= 0 && bi == sbid[j])
+      up = tk.blocks[bi].acc[sbpos[i] + static_cast<size_t>(tk.blocks[bi].size) * sbpos[j]];
+    tk.acc[i + static_cast<size_t>(k) * j] = v + up;
+  });
 }
 
 __global__ void assemble_top_kernel(int pde, const Node* nodes, const int* dofs, int n,
@@ -225,21 +442,41 @@ cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* s
   return cudaGetLastError();
 }
 
-size_t decouple_smem_bytes(int n_max) {
-  const int ns = n_max < kSmemN ? n_max : kSmemN;
-  return sizeof(double) * (kGemmTileDoubles + 64 + static_cast<size_t>(ns) * ns);
-}
-
-cudaError_t launch_decouple(const DecParams& p, int n_max, cudaStream_t s) {
-  if (p.ntasks == 0) return cudaSuccess;
-  const size_t smem = decouple_smem_bytes(n_max);
-  cudaError_t e = raise_func_attr(reinterpret_cast<const void*>(&decouple_kernel),
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+namespace {
+// The register tile of X_rr's inversion by r, and the CTAs of it an SM's
+// registers hold.
+template <int CW, int RS, int MINB>
+cudaError_t launch_class(const DecParams& p, bool fast, size_t smem, cudaStream_t s) {
+  const void* fn = fast ? reinterpret_cast<const void*>(&decouple_kernel<CW, RS, MINB, true>)
+                        : reinterpret_cast<const void*>(&decouple_kernel<CW, RS, MINB, false>);
+  cudaError_t e = raise_func_attr(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   count_launches(1);
-  decouple_kernel<<<p.ntasks, kDecThreads, smem, s>>>(p);
+  if (fast) {
+    decouple_kernel<CW, RS, MINB, true><<<p.ntasks, kDecThreads, smem, s>>>(p);
+  } else {
+    decouple_kernel<CW, RS, MINB, false><<<p.ntasks, kDecThreads, smem, s>>>(p);
+  }
   return cudaGetLastError();
+}
+}  // namespace
+
+size_t decouple_smem_bytes(int n, int k, bool fast) { return dec_layout(n, k, !fast).bytes; }
+
+int decouple_class(int n, int k) {
+  const int r = n - k;
+  return r <= 64 ? 0 : r <= 96 ? 1 : r <= 160 ? 2 : -1;
+}
+
+cudaError_t launch_decouple(const DecParams& p, int cls, bool fast, size_t smem, cudaStream_t s) {
+  if (p.ntasks == 0) return cudaSuccess;
+  switch (cls) {
+    case 0: return launch_class<8, 2, 3>(p, fast, smem, s);
+    case 1: return launch_class<12, 3, 2>(p, fast, smem, s);
+    case 2: return launch_class<20, 5, 1>(p, fast, smem, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 cudaError_t launch_assemble_top(int pde, const Node* nodes, const int* dofs, int n,

@@ -158,12 +158,14 @@ struct DecParams {
   int* status;  // set nonzero on an exactly zero pivot
 };
 
-// n_max: largest box of the launch (sizes the shared-memory staging).
-// Boxes with n > kDecoupleSmemN must go through decouple_large instead.
-constexpr int kDecoupleSmemN = 160;
-cudaError_t launch_decouple(const DecParams& p, int n_max, cudaStream_t s);
-// Dynamic shared memory of a decouple launch whose largest box has n_max dofs.
-size_t decouple_smem_bytes(int n_max);
+// One launch for boxes of one class (decouple_class: the size of X_rr's
+// register tile; -1: too large for a CTA) with `smem` bytes, the largest
+// decouple_smem_bytes of them.  fast: contracted entries, L not corrected (a
+// preconditioner's).  Boxes of class -1 or past 227 KB go through
+// decouple_large instead.
+int decouple_class(int n, int k);
+size_t decouple_smem_bytes(int n, int k, bool fast);
+cudaError_t launch_decouple(const DecParams& p, int cls, bool fast, size_t smem, cudaStream_t s);
 // The same decoupling for one large box as a sequence of GPU-wide kernels
 // (tk is the host copy of the box's descriptor; tk.K must hold n x n).
 cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* status,

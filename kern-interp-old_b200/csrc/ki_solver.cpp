@@ -715,15 +715,18 @@ int Solver::finish_factor(cudaEvent_t ev0) {
     for (int level = L - 1; level > 0 && !rc; level--) {
       auto next = std::make_unique<PendingLevel>();
       const bool more = level > 1 && !(level == 2 && level1_stays());
-      // what the factorization waits for goes first: the decouplings of a
-      // preconditioner (measured on a B200: see the stream priorities), the
-      // IDs of a reference factorization
-      if (opt_.sketch_id) rc = decouple_level(cur.get());
+      // the deepest level's decouplings, when they fill the GPU more than
+      // once, are the head of the chain a preconditioner's factorization
+      // waits for: queued before the next IDs are prepared (every later
+      // level's wait for the ones below in any case)
+      const bool dec_first = opt_.sketch_id && level == L - 1 &&
+                             static_cast<int>(cur->comp.size()) > 2 * num_sms_;
+      if (dec_first) rc = decouple_level(cur.get());
       if (!rc && more) {
         rc = id_launch(level - 1, next.get());
         refreshed = level - 1;
       }
-      if (!rc && !opt_.sketch_id) rc = decouple_level(cur.get());
+      if (!rc && !dec_first) rc = decouple_level(cur.get());
       if (!rc && more) rc = id_finish(next.get());
       if (!more) break;
       cur = std::move(next);
@@ -1268,6 +1271,10 @@ int Solver::decouple_boxes(PendingLevel* pl) {
       }
     }
   });
+  const bool fast = opt_.sketch_id;
+  auto large_box = [&](int n, int k) {
+    return decouple_class(n, k) < 0 || decouple_smem_bytes(n, k, fast) > 227 * 1024;
+  };
   std::vector<long long> bid_off(ncomp + 1, 0), tab_off(ncomp + 1, 0);
   long long scratch_total = 0;
   std::vector<long long> k_off(ncomp), x0_off(ncomp);
@@ -1280,7 +1287,7 @@ int Solver::decouple_boxes(PendingLevel* pl) {
     bid_off[t + 1] = bid_off[t] + n;
     tab_off[t + 1] = tab_off[t] + static_cast<long long>(blk[t].size());
     k_off[t] = scratch_total;
-    if (n > kDecoupleSmemN) {
+    if (large_box(n, k)) {
       // n x n, then the LU's flags (kLuSyncInts ints)
       scratch_total += static_cast<long long>(n) * n + kLuSyncInts;
     } else {
@@ -1366,10 +1373,19 @@ int Solver::decouple_boxes(PendingLevel* pl) {
   }
   // small boxes first in one batched launch, then each large box
   std::vector<DecTask> small, large;
-  for (const DecTask& d : dt) (d.n > kDecoupleSmemN ? large : small).push_back(d);
-  // the largest boxes first (CTAs start in index order: no long last wave)
-  std::stable_sort(small.begin(), small.end(),
-                   [](const DecTask& a, const DecTask& b) { return a.n > b.n; });
+  for (const DecTask& d : dt) (large_box(d.n, d.k) ? large : small).push_back(d);
+  // by launch (class, then how many CTAs' shared memory an SM holds, three at
+  // most: 1 KB of each CTA's is reserved by the system), the largest boxes
+  // first in each (CTAs start in index order: no long last wave)
+  auto launch_key = [&](const DecTask& d) {
+    const size_t bytes = decouple_smem_bytes(d.n, d.k, fast) + 1024;
+    return 4 * decouple_class(d.n, d.k) +
+           3 - static_cast<int>(std::min<size_t>(3, static_cast<size_t>(smem_per_sm_) / bytes));
+  };
+  std::stable_sort(small.begin(), small.end(), [&](const DecTask& a, const DecTask& b) {
+    const int ka = launch_key(a), kb = launch_key(b);
+    return ka != kb ? ka > kb : a.n > b.n;
+  });
   KI_UPLOAD(d_bid, bid, ustream_);
   KI_UPLOAD(d_bpos, bpos, ustream_);
   KI_UPLOAD(d_tab, tab, ustream_);
@@ -1386,13 +1402,10 @@ int Solver::decouple_boxes(PendingLevel* pl) {
   t_host_post_ms += now_ms() - h1;
   mark(3, level);
   if (time_phases && timer_begin(&d0, dstream_)) return -2;
-  // The batched boxes in size classes, one launch each: a launch's shared
-  // memory is sized by its largest box, so the boxes of a level are grouped
-  // by how many CTAs of theirs an SM holds (three at most: 72 registers x
-  // 256 threads; on a B200 n <= 85 gives three, n <= 110 two); the widest
-  // class on dstream_, the others and the large boxes (one multi-kernel
-  // sequence each) side by side on their own streams after the level's
-  // uploads, joined back into dstream_.
+  // The batched boxes, one launch per key (a launch's registers and shared
+  // memory are sized by its largest box); the first on dstream_, the others
+  // and the large boxes (one multi-kernel sequence each) side by side on
+  // their own streams after the level's uploads, joined back into dstream_.
   KI_CUDA(cudaEventRecord(dl_fork_, dstream_));
   bool used[kDecStreams] = {};
   int next_side = 0;
@@ -1405,19 +1418,19 @@ int Solver::decouple_boxes(PendingLevel* pl) {
     *out = dl_streams_[si];
     return 0;
   };
-  auto size_class = [&](int n) {
-    // (1 KB of each CTA's shared memory is reserved by the system)
-    return std::min<size_t>(3, static_cast<size_t>(smem_per_sm_) / (decouple_smem_bytes(n) + 1024));
-  };
   for (size_t a = 0; a < small.size();) {
-    size_t b = a;
-    while (b < small.size() && size_class(small[b].n) == size_class(small[a].n)) b++;
+    size_t b = a, smem = 0;
+    const int key = launch_key(small[a]);
+    while (b < small.size() && launch_key(small[b]) == key) {
+      smem = std::max(smem, decouple_smem_bytes(small[b].n, small[b].k, fast));
+      b++;
+    }
     DecParams dpc = dp;
     dpc.tasks = d_dt + a;
     dpc.ntasks = static_cast<int>(b - a);
     cudaStream_t cs = dstream_;
     if (a > 0 && side_stream(&cs)) return -2;
-    KI_CUDA(launch_decouple(dpc, small[a].n, cs));  // (sorted: the class's largest first)
+    KI_CUDA(launch_decouple(dpc, key / 4, fast, smem, cs));
     a = b;
   }
   int n_large = 0;
