@@ -350,7 +350,9 @@ cudaError_t launch_eval_targets(int pde, const Node* nodes, int n_dofs, int nt,
 // linear_solve.cpp:142-180).  kind: kDomainAll (no mask), kDomainNodes
 // (CubicBoundary::is_in_domain on the node curves), kDomainDisk (the
 // Circle / Annulus / Donut test with disk = {cx, cy, R}).  mask: 1 inside,
-// 0 outside.  launch_domain_eval zeroes outside points when mask is given;
+// 0 outside.  inside, if given (1 + nt ints), receives the number of points
+// inside and their list; launch_domain_eval zeroes outside points when mask
+// is given, with the list of the others, whose sums alone it forms;
 // `part` holds splits x rows doubles when splits > 1 (domain_splits).
 enum DomainKind : int { kDomainAll = 0, kDomainNodes = 1, kDomainDisk = 2 };
 int domain_splits(int nt, int np, int num_sms);
@@ -358,12 +360,13 @@ int domain_splits(int nt, int np, int num_sms);
 size_t domain_mask_scratch_bytes(int np);
 cudaError_t launch_domain_mask(int kind, const Node* nodes, int np, const double* holes, int nh,
                                const double* disk, int nt, const double* targets,
-                               unsigned char* mask, void* scratch, cudaStream_t s);
+                               unsigned char* mask, int* inside, void* scratch,
+                               cudaStream_t s);
 cudaError_t launch_domain_eval(int pde, const Node* nodes, int np, int nt,
                                const double* targets, const double* mu, int nh,
                                const double* holes, const double* alpha,
-                               const unsigned char* mask, int splits, double* part,
-                               double* out, cudaStream_t s);
+                               const unsigned char* mask, const int* inside, int splits,
+                               double* part, double* out, cudaStream_t s);
 // cudaFuncSetAttribute(func, attr, value) unless this process already
 // raised the attribute to at least `value` on the current device: the call
 // costs microseconds of host time, which level loops with many short
