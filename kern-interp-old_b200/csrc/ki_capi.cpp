@@ -2,6 +2,8 @@
 // include/kinterp.h).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -11,6 +13,7 @@
 
 #include "../../include/kinterp.h"
 #include "ki_kernels.h"
+#include "ki_pool.h"
 #include "ki_solver.h"
 
 struct ki_solver_s {
@@ -93,9 +96,15 @@ bool box_ref(ki_solver_t s, int level, int idx, const kib::Box** out, int* paren
 // Every value finite (NaN and infinities fail): boundary data with a
 // non-finite value would only surface as NaN factors.
 bool all_finite(const double* a, size_t n) {
-  bool ok = true;
-  for (size_t i = 0; i < n; i++) ok &= std::isfinite(a[i]);
-  return ok;
+  constexpr size_t kChunk = 1 << 15;
+  std::atomic<bool> ok{true};
+  kib::parallel_for(static_cast<int>((n + kChunk - 1) / kChunk), 1, [&](int b, int e) {
+    bool fin = true;
+    for (size_t i = b * kChunk, end = std::min(n, e * kChunk); i < end; i++)
+      fin &= std::isfinite(a[i]);
+    if (!fin) ok.store(false);
+  }, 3);
+  return ok.load();
 }
 
 bool geometry_finite(int n_points, const double* points, const double* normals,

@@ -207,6 +207,23 @@ template int Solver::upload<int>(int*, const std::vector<int>&, cudaStream_t);
 template int Solver::upload<double>(double*, const std::vector<double>&, cudaStream_t);
 template int Solver::upload<MvTile>(MvTile*, const std::vector<MvTile>&, cudaStream_t);
 
+void Solver::set_geometry(const double* points, const double* normals, const double* curvatures,
+                          const double* weights) {
+  const size_t n = static_cast<size_t>(n_points_);
+  pts_.resize(2 * n);
+  nrm_.resize(2 * n);
+  curv_.resize(n);
+  wts_.resize(n);
+  // (the copies' first touch of fresh pages is most of their cost)
+  parallel_for(n_points_, 8192, [&](int a, int e) {
+    const size_t c = static_cast<size_t>(e) - a, o = static_cast<size_t>(a);
+    std::memcpy(pts_.data() + 2 * o, points + 2 * o, 2 * c * sizeof(double));
+    std::memcpy(nrm_.data() + 2 * o, normals + 2 * o, 2 * c * sizeof(double));
+    std::memcpy(curv_.data() + o, curvatures + o, c * sizeof(double));
+    std::memcpy(wts_.data() + o, weights + o, c * sizeof(double));
+  }, 16384);
+}
+
 Solver::Solver(const SolverOptions& opt, int n_points, const double* points,
                const double* normals, const double* curvatures, const double* weights,
                int n_holes, const double* holes, cudaStream_t stream)
@@ -214,10 +231,7 @@ Solver::Solver(const SolverOptions& opt, int n_points, const double* points,
   sd_ = opt.pde == kStokes ? 2 : 1;
   n_points_ = n_points;
   n_dofs_ = n_points * sd_;
-  pts_.assign(points, points + 2 * static_cast<size_t>(n_points));
-  nrm_.assign(normals, normals + 2 * static_cast<size_t>(n_points));
-  curv_.assign(curvatures, curvatures + n_points);
-  wts_.assign(weights, weights + n_points);
+  set_geometry(points, normals, curvatures, weights);
   if (n_holes > 0) holes_.assign(holes, holes + 4 * static_cast<size_t>(n_holes));
 }
 
@@ -384,37 +398,35 @@ int Solver::cuda_check(cudaError_t e, const char* what) {
   return -2;
 }
 
-std::vector<BoxBlock> Solver::blocks_of(int box) const {
-  // Accumulated updates inside the box's current dof list: its own skeleton
-  // update when compressed, else its children's lists laid end to end.
+void Solver::child_blocks(int box, int off, std::vector<BoxBlock>* out) const {
+  // Accumulated updates inside the box's dof list, which starts at off: its
+  // children's lists laid end to end, of a compressed child its own skeleton
+  // update.
   const Box& b = tree.boxes[box];
-  if (b.compressed) return {BoxBlock{boxdev_[box].acc, b.rank, 0}};
-  std::vector<BoxBlock> out;
-  if (b.leaf) return out;
-  int off = 0;
+  if (b.leaf) return;
   for (int q = 0; q < 4; q++) {
     const int c = b.child[q];
-    for (const BoxBlock& x : blocks_of(c)) out.push_back(BoxBlock{x.acc, x.size, x.pos + off});
     const Box& cb = tree.boxes[c];
+    if (cb.compressed) {
+      out->push_back(BoxBlock{boxdev_[c].acc, cb.rank, off});
+    } else {
+      child_blocks(c, off, out);
+    }
     off += static_cast<int>(cb.compressed ? cb.skel.size() : cb.active.size());
   }
-  return out;
 }
 
-void Solver::build_block_map(const std::vector<BoxBlock>& blocks, int n, std::vector<int>* bid,
-                             std::vector<int>* bpos, std::vector<UpdBlock>* tab) const {
-  const int base = static_cast<int>(tab->size());
-  const size_t b0 = bid->size();
-  bid->resize(b0 + n, -1);
-  bpos->resize(b0 + n, 0);
+void Solver::fill_block_map(const std::vector<BoxBlock>& blocks, int n, int* bid, int* bpos,
+                            UpdBlock* tab) {
+  std::fill(bid, bid + n, -1);
+  std::fill(bpos, bpos + n, 0);
   for (size_t q = 0; q < blocks.size(); q++) {
-    tab->push_back(UpdBlock{blocks[q].acc, blocks[q].size, 0});
+    tab[q] = UpdBlock{blocks[q].acc, blocks[q].size, 0};
     for (int t = 0; t < blocks[q].size; t++) {
-      (*bid)[b0 + blocks[q].pos + t] = static_cast<int>(q);
-      (*bpos)[b0 + blocks[q].pos + t] = t;
+      bid[blocks[q].pos + t] = static_cast<int>(q);
+      bpos[blocks[q].pos + t] = t;
     }
   }
-  (void)base;
 }
 
 void Solver::build_tree_only() {
@@ -430,7 +442,7 @@ void Solver::build_tree_only() {
 }
 
 void Solver::perturb_tree_only(int n_points, const double* points) {
-  const std::vector<double> old = pts_;
+  const HostArray old = pts_;
   const int n_old = n_points_;
   n_points_ = n_points;
   n_dofs_ = n_points * sd_;
@@ -873,18 +885,18 @@ int Solver::id_launch(int level, PendingLevel* pl) {
     }
   });
   mark(10, level);
-  std::vector<Cand>& cand = pl->cand;
+  std::vector<int> order;
   for (int q = 0; q < nids; q++)
-    if (keep[q]) cand.push_back(std::move(all[q]));
-  if (cand.empty()) return 0;
+    if (keep[q]) order.push_back(q);
+  if (order.empty()) return 0;
   // A box in registers takes more CTAs than one in shared memory (160 KB of
   // an SM's registers hold matrix entries, 220 KB of its shared memory) but
   // is done sooner, so a level that fits the GPU in registers takes them and
   // a fuller one the smaller clusters.
   int ctas = 0;
-  for (const Cand& c : cand) ctas += c.g % 100;
+  for (int q : order) ctas += all[q].g % 100;
   if (ctas > num_sms_)
-    for (Cand& c : cand)
+    for (Cand& c : all)
       if (c.g_slab && c.g >= kTile && c.g_slab % 100 < c.g % 100) c.g = c.g_slab;
   // grouped by cluster size, the group holding the widest ID matrix first
   // (its launch then takes SMs before the many-box launch fills them: the
@@ -892,11 +904,13 @@ int Solver::id_launch(int level, PendingLevel* pl) {
   // largest first (CTAs start in index order, so the long tasks do not end
   // up in a launch's last wave)
   std::map<int, long long> group_max;  // widest task (its steps and sketch rows grow with n)
-  for (const Cand& c : cand) {
+  for (int q : order) {
+    const Cand& c = all[q];
     long long& v = group_max[c.g];
     v = std::max(v, static_cast<long long>(c.n) * 100000 + std::min(c.m, 99999));
   }
-  std::stable_sort(cand.begin(), cand.end(), [&](const Cand& a, const Cand& b) {
+  std::stable_sort(order.begin(), order.end(), [&](int qa, int qb) {
+    const Cand &a = all[qa], &b = all[qb];
     if (a.g != b.g) {
       const long long ma = group_max[a.g], mb = group_max[b.g];
       return ma != mb ? ma > mb : a.g > b.g;
@@ -905,7 +919,12 @@ int Solver::id_launch(int level, PendingLevel* pl) {
   });
 
   mark(11, level);
-  const int nc = static_cast<int>(cand.size());
+  const int nc = static_cast<int>(order.size());
+  std::vector<Cand>& cand = pl->cand;
+  cand.resize(nc);
+  parallel_for(nc, 64, [&](int a, int e) {
+    for (int q = a; q < e; q++) cand[q] = std::move(all[order[q]]);
+  }, 512);
   std::vector<IdTask>& tasks = pl->tasks;
   tasks.assign(nc, IdTask{});
   long long a_total = 0, t_total = 0;
@@ -933,10 +952,20 @@ int Solver::id_launch(int level, PendingLevel* pl) {
     t_total += static_cast<long long>(c.n) * c.n / 4 + 1;
     perm_total += c.n;
   }
-  std::vector<int> act(act_total), rows(rows_total);
+  // the level's three lists in one host-to-device copy (formed in its pinned
+  // staging) and its ranks and pivots in one copy back: each copy adds its own
+  // latency to the chain of ID levels (a level's lists wait for the ranks of
+  // the level below)
+  const size_t o_rows = (sizeof(int) * act_total + 255) & ~static_cast<size_t>(255);
+  const size_t o_tasks = o_rows + ((sizeof(int) * rows_total + 255) & ~static_cast<size_t>(255));
+  const size_t b_pack = o_tasks + sizeof(IdTask) * nc;
+  char* st = static_cast<char*>(stage_.alloc(b_pack));
+  if (!st) return fail("pinned staging allocation failed");
+  int* act = reinterpret_cast<int*>(st);
+  int* rows = reinterpret_cast<int*>(st + o_rows);
   parallel_for(nc, 16, [&](int a, int e) {  // descriptors and lists
     for (int q = a; q < e; q++) {
-      const Cand& c = cand[q];
+      Cand& c = cand[q];
       const Box& b = tree.boxes[c.box];
       IdTask& t = tasks[q];
       t.n = c.n;
@@ -949,22 +978,17 @@ int Solver::id_launch(int level, PendingLevel* pl) {
       t.cy = b.corner[1] + b.side / 2.0;
       t.rad = b.side * kRadiusRatio;
       t.pw = 2.0 * M_PI * t.rad / (kNumProxy >> t.pshift);
-      std::copy(b.active.begin(), b.active.end(), act.begin() + t.act_off);
-      std::copy(c.rows.begin(), c.rows.end(), rows.begin() + t.row_off);
+      std::copy(b.active.begin(), b.active.end(), act + t.act_off);
+      std::copy(c.rows.begin(), c.rows.end(), rows + t.row_off);
+      std::vector<int>().swap(c.rows);
     }
   });
+  std::memcpy(st + o_tasks, tasks.data(), sizeof(IdTask) * nc);
   t_host_prep_ms += now_ms() - h0;
   mark(1, level);
   int *d_act, *d_rows, *d_perm, *d_rank;
   double* d_T;
   IdTask* d_tasks;
-  // the level's three lists in one host-to-device copy and its ranks and
-  // pivots in one copy back: each copy adds its own latency to the chain of
-  // ID levels (a level's lists wait for the ranks of the level below)
-  const size_t b_act = sizeof(int) * act.size(), b_rows = sizeof(int) * rows.size();
-  const size_t o_rows = (b_act + 255) & ~static_cast<size_t>(255);
-  const size_t o_tasks = o_rows + ((b_rows + 255) & ~static_cast<size_t>(255));
-  const size_t b_pack = o_tasks + sizeof(IdTask) * nc;
   char* d_pack;
   KI_ALLOC(d_pack, char, b_pack);
   d_act = reinterpret_cast<int*>(d_pack);
@@ -974,14 +998,7 @@ int Solver::id_launch(int level, PendingLevel* pl) {
   d_perm = d_rank + nc;
   KI_ALLOC(d_T, double, t_total);
   KI_CUDA(work_.reserve(sizeof(double) * a_total, stream_));
-  {
-    char* st = static_cast<char*>(stage_.alloc(b_pack));
-    if (!st) return fail("pinned staging allocation failed");
-    if (b_act) std::memcpy(st, act.data(), b_act);
-    if (b_rows) std::memcpy(st + o_rows, rows.data(), b_rows);
-    std::memcpy(st + o_tasks, tasks.data(), sizeof(IdTask) * nc);
-    KI_CUDA(cudaMemcpyAsync(d_pack, st, b_pack, cudaMemcpyHostToDevice, stream_));
-  }
+  KI_CUDA(cudaMemcpyAsync(d_pack, st, b_pack, cudaMemcpyHostToDevice, stream_));
 
   // one launch per cluster size (split further so that the launch's
   // shared-memory layout, sized by its largest rows / columns / column
@@ -1254,21 +1271,12 @@ int Solver::decouple_boxes(PendingLevel* pl) {
   int* d_act = pl->d_act;
   int* d_perm = pl->d_perm;
   const int ncomp = static_cast<int>(comp.size());
-  std::vector<DecTask> dt(ncomp);
   // block maps (per position of the box's dof list: which descendant
   // update, and where in it), made per box in parallel at precomputed offsets
   std::vector<std::vector<BoxBlock>> blk(ncomp);
   parallel_for(ncomp, 16, [&](int a, int e) {
     for (int t = a; t < e; t++) {
-      const Box& b = tree.boxes[cand[comp[t]].box];
-      if (b.leaf) continue;
-      int off = 0;
-      for (int q = 0; q < 4; q++) {
-        const int ch = b.child[q];
-        for (const BoxBlock& x : blocks_of(ch)) blk[t].push_back(BoxBlock{x.acc, x.size, x.pos + off});
-        const Box& cb = tree.boxes[ch];
-        off += static_cast<int>(cb.compressed ? cb.skel.size() : cb.active.size());
-      }
+      child_blocks(cand[comp[t]].box, 0, &blk[t]);
     }
   });
   const bool fast = opt_.sketch_id;
@@ -1278,6 +1286,7 @@ int Solver::decouple_boxes(PendingLevel* pl) {
   std::vector<long long> bid_off(ncomp + 1, 0), tab_off(ncomp + 1, 0);
   long long scratch_total = 0;
   std::vector<long long> k_off(ncomp), x0_off(ncomp);
+  std::vector<size_t> f_off(ncomp), p_off(ncomp);
   int n_max = 0;
   size_t fac_total = 0, piv_total = 0;
   for (int t = 0; t < ncomp; t++) {
@@ -1295,6 +1304,8 @@ int Solver::decouple_boxes(PendingLevel* pl) {
     }
     x0_off[t] = scratch_total;
     if (!opt_.sketch_id) scratch_total += static_cast<long long>(r) * r;
+    f_off[t] = fac_total;
+    p_off[t] = piv_total;
     fac_total += static_cast<size_t>(k) * r * 2 + static_cast<size_t>(r) * r +
                  static_cast<size_t>(k) * k;
     piv_total += r;
@@ -1307,94 +1318,89 @@ int Solver::decouple_boxes(PendingLevel* pl) {
       solve_bytes += 8.0 * (4.0 * dk * dr + dr * dr);
     }
   }
-  std::vector<int> bid(bid_off[ncomp], -1), bpos(bid_off[ncomp], 0);
-  std::vector<UpdBlock> tab(tab_off[ncomp]);
-  parallel_for(ncomp, 16, [&](int a, int e) {
-    for (int t = a; t < e; t++) {
-      const std::vector<BoxBlock>& bl = blk[t];
-      int* bi = bid.data() + bid_off[t];
-      int* bp = bpos.data() + bid_off[t];
-      for (size_t q = 0; q < bl.size(); q++) {
-        tab[tab_off[t] + q] = UpdBlock{bl[q].acc, bl[q].size, 0};
-        for (int u = 0; u < bl[q].size; u++) {
-          bi[bl[q].pos + u] = static_cast<int>(q);
-          bp[bl[q].pos + u] = u;
-        }
-      }
-    }
-  });
-  int *d_bid, *d_bpos, *d_piv;
-  UpdBlock* d_tab;
+  int* d_piv;
   double* d_fac;
-  DecTask* d_dt;
-  KI_ALLOC(d_bid, int, bid.size());
-  KI_ALLOC(d_bpos, int, bpos.size());
-  KI_ALLOC(d_tab, UpdBlock, tab.size());
   KI_ALLOC(d_fac, double, fac_total);
   KI_ALLOC(d_piv, int, piv_total);
-  KI_ALLOC(d_dt, DecTask, ncomp);
   // (earlier levels' decouplings may still be queued on dstream_ with the
   // old buffer: it is retired, not waited for)
   KI_CUDA(scratch2_.reserve(sizeof(double) * (scratch_total + 1), dstream_, true));
   double* scr = static_cast<double*>(scratch2_.p);
-  size_t fo = 0, po = 0;
+  // small boxes in batched launches, by launch (class, then how many CTAs'
+  // shared memory an SM holds, three at most: 1 KB of each CTA's is reserved
+  // by the system), the largest boxes first in each (CTAs start in index
+  // order: no long last wave); then each large box on its own
+  std::vector<int> key(ncomp), small, large;
   for (int t = 0; t < ncomp; t++) {
-    const Cand& c = cand[comp[t]];
-    const IdTask& it = tasks[comp[t]];
-    const Box& b = tree.boxes[c.box];
-    const int n = c.n, k = b.rank, r = n - k;
-    BoxDev& bd = boxdev_[c.box];
-    bd.L = d_fac + fo;
-    fo += static_cast<size_t>(k) * r;
-    bd.U = d_fac + fo;
-    fo += static_cast<size_t>(k) * r;
-    bd.X = d_fac + fo;
-    fo += static_cast<size_t>(r) * r;
-    bd.acc = d_fac + fo;
-    fo += static_cast<size_t>(k) * k;
-    bd.piv = d_piv + po;
-    po += r;
-    DecTask& d = dt[t];
-    d.n = n;
-    d.k = k;
-    d.act = d_act + it.act_off;
-    d.perm = d_perm + it.perm_off;
-    d.bid = d_bid + bid_off[t];
-    d.bpos = d_bpos + bid_off[t];
-    d.blocks = d_tab + tab_off[t];
-    d.T = bd.T;
-    d.K = scr + k_off[t];
-    d.L = bd.L;
-    d.U = bd.U;
-    d.X = bd.X;
-    d.acc = bd.acc;
-    d.piv = bd.piv;
-    d.X0 = opt_.sketch_id ? nullptr : scr + x0_off[t];
+    const int n = cand[comp[t]].n, k = tree.boxes[cand[comp[t]].box].rank;
+    if (large_box(n, k)) {
+      large.push_back(t);
+      continue;
+    }
+    const size_t bytes = decouple_smem_bytes(n, k, fast) + 1024;
+    key[t] = 4 * decouple_class(n, k) +
+             3 - static_cast<int>(std::min<size_t>(3, static_cast<size_t>(smem_per_sm_) / bytes));
+    small.push_back(t);
   }
-  // small boxes first in one batched launch, then each large box
-  std::vector<DecTask> small, large;
-  for (const DecTask& d : dt) (large_box(d.n, d.k) ? large : small).push_back(d);
-  // by launch (class, then how many CTAs' shared memory an SM holds, three at
-  // most: 1 KB of each CTA's is reserved by the system), the largest boxes
-  // first in each (CTAs start in index order: no long last wave)
-  auto launch_key = [&](const DecTask& d) {
-    const size_t bytes = decouple_smem_bytes(d.n, d.k, fast) + 1024;
-    return 4 * decouple_class(d.n, d.k) +
-           3 - static_cast<int>(std::min<size_t>(3, static_cast<size_t>(smem_per_sm_) / bytes));
-  };
-  std::stable_sort(small.begin(), small.end(), [&](const DecTask& a, const DecTask& b) {
-    const int ka = launch_key(a), kb = launch_key(b);
-    return ka != kb ? ka > kb : a.n > b.n;
+  std::stable_sort(small.begin(), small.end(), [&](int a, int b) {
+    return key[a] != key[b] ? key[a] > key[b] : cand[comp[a]].n > cand[comp[b]].n;
   });
-  KI_UPLOAD(d_bid, bid, ustream_);
-  KI_UPLOAD(d_bpos, bpos, ustream_);
-  KI_UPLOAD(d_tab, tab, ustream_);
-  KI_UPLOAD(d_dt, small, ustream_);
+  const int nsmall = static_cast<int>(small.size());
+  std::vector<int> at(small);  // place of a box: small ones, then large ones
+  at.insert(at.end(), large.begin(), large.end());
+  std::vector<DecTask> dt(ncomp);
+  // one staging block and one copy: [tasks | update blocks | block of each
+  // position | place in it]
+  const size_t o_tab = sizeof(DecTask) * nsmall;
+  const size_t o_ints = o_tab + sizeof(UpdBlock) * tab_off[ncomp];
+  const size_t b_pack = o_ints + 2 * sizeof(int) * bid_off[ncomp];
+  char *d_pack, *st = static_cast<char*>(stage_.alloc(b_pack + 16));
+  if (!st) return fail("pinned staging allocation failed");
+  KI_ALLOC(d_pack, char, b_pack + 16);
+  DecTask* d_dt = reinterpret_cast<DecTask*>(d_pack);
+  UpdBlock* d_tab = reinterpret_cast<UpdBlock*>(d_pack + o_tab);
+  int* d_bid = reinterpret_cast<int*>(d_pack + o_ints);
+  int* d_bpos = d_bid + bid_off[ncomp];
+  parallel_for(ncomp, 16, [&](int a, int e) {
+    int* hb = reinterpret_cast<int*>(st + o_ints);
+    for (int i = a; i < e; i++) {
+      const int t = at[i];
+      const Cand& c = cand[comp[t]];
+      const IdTask& it = tasks[comp[t]];
+      const int n = c.n, k = tree.boxes[c.box].rank, r = n - k;
+      fill_block_map(blk[t], n, hb + bid_off[t], hb + bid_off[ncomp] + bid_off[t],
+                     reinterpret_cast<UpdBlock*>(st + o_tab) + tab_off[t]);
+      BoxDev& bd = boxdev_[c.box];
+      bd.L = d_fac + f_off[t];
+      bd.U = bd.L + static_cast<size_t>(k) * r;
+      bd.X = bd.U + static_cast<size_t>(k) * r;
+      bd.acc = bd.X + static_cast<size_t>(r) * r;
+      bd.piv = d_piv + p_off[t];
+      DecTask& d = dt[i];
+      d.n = n;
+      d.k = k;
+      d.act = d_act + it.act_off;
+      d.perm = d_perm + it.perm_off;
+      d.bid = d_bid + bid_off[t];
+      d.bpos = d_bpos + bid_off[t];
+      d.blocks = d_tab + tab_off[t];
+      d.T = bd.T;
+      d.K = scr + k_off[t];
+      d.L = bd.L;
+      d.U = bd.U;
+      d.X = bd.X;
+      d.acc = bd.acc;
+      d.piv = bd.piv;
+      d.X0 = opt_.sketch_id ? nullptr : scr + x0_off[t];
+      if (i < nsmall) reinterpret_cast<DecTask*>(st)[i] = d;
+    }
+  });
+  KI_CUDA(cudaMemcpyAsync(d_pack, st, b_pack, cudaMemcpyHostToDevice, ustream_));
   KI_CUDA(cudaEventRecord(ev_up_, ustream_));
   KI_CUDA(cudaStreamWaitEvent(dstream_, ev_up_, 0));
   DecParams dp{};
   dp.tasks = d_dt;
-  dp.ntasks = static_cast<int>(small.size());
+  dp.ntasks = nsmall;
   dp.pde = opt_.pde;
   dp.nodes = d_nodes_;
   dp.status = d_status_;
@@ -1418,27 +1424,28 @@ int Solver::decouple_boxes(PendingLevel* pl) {
     *out = dl_streams_[si];
     return 0;
   };
-  for (size_t a = 0; a < small.size();) {
-    size_t b = a, smem = 0;
-    const int key = launch_key(small[a]);
-    while (b < small.size() && launch_key(small[b]) == key) {
-      smem = std::max(smem, decouple_smem_bytes(small[b].n, small[b].k, fast));
+  for (int a = 0; a < nsmall;) {
+    int b = a;
+    size_t smem = 0;
+    const int ka = key[small[a]];
+    while (b < nsmall && key[small[b]] == ka) {
+      smem = std::max(smem, decouple_smem_bytes(dt[b].n, dt[b].k, fast));
       b++;
     }
     DecParams dpc = dp;
     dpc.tasks = d_dt + a;
-    dpc.ntasks = static_cast<int>(b - a);
+    dpc.ntasks = b - a;
     cudaStream_t cs = dstream_;
     if (a > 0 && side_stream(&cs)) return -2;
-    KI_CUDA(launch_decouple(dpc, key / 4, fast, smem, cs));
+    KI_CUDA(launch_decouple(dpc, ka / 4, fast, smem, cs));
     a = b;
   }
   int n_large = 0;
-  for (size_t t = 0; t < large.size(); t++) {
+  for (int t = nsmall; t < ncomp; t++) {
     cudaStream_t cs;
     if (side_stream(&cs)) return -2;
-    KI_CUDA(decouple_large(large[t], opt_.pde, d_nodes_, d_status_, cs));
-    n_large = std::max(n_large, large[t].n);
+    KI_CUDA(decouple_large(dt[t], opt_.pde, d_nodes_, d_status_, cs));
+    n_large = std::max(n_large, dt[t].n);
   }
   for (int i = 0; i < kDecStreams; i++)
     if (used[i]) {
@@ -1460,37 +1467,45 @@ int Solver::level_sweeps(int level, const std::vector<int>& boxes, cudaStream_t 
   lf.level = level;
   const int ncomp = static_cast<int>(boxes.size());
   if (ncomp == 0) return 0;
-  std::vector<int> sk, rd;
-  std::vector<SweepTask> st(ncomp);
-  std::vector<int> sk_off(ncomp), rd_off(ncomp);
+  std::vector<int> sk_off(ncomp + 1, 0), rd_off(ncomp + 1, 0);
   int cap = 0, kr = 0;
   for (int t = 0; t < ncomp; t++) {
     const Box& b = tree.boxes[boxes[t]];
-    sk_off[t] = static_cast<int>(sk.size());
-    rd_off[t] = static_cast<int>(rd.size());
-    sk.insert(sk.end(), b.skel.begin(), b.skel.end());
-    rd.insert(rd.end(), b.redundant.begin(), b.redundant.end());
-    cap = std::max(cap, static_cast<int>(b.skel.size() + b.redundant.size()));
-    kr = std::max(kr, static_cast<int>(b.skel.size() * b.redundant.size()));
-    lf.boxes.push_back(boxes[t]);
+    const int ks = static_cast<int>(b.skel.size()), r = static_cast<int>(b.redundant.size());
+    sk_off[t + 1] = sk_off[t] + ks;
+    rd_off[t + 1] = rd_off[t] + r;
+    cap = std::max(cap, ks + r);
+    kr = std::max(kr, ks * r);
   }
-  KI_ALLOC(lf.d_skel, int, sk.size());
-  KI_ALLOC(lf.d_red, int, rd.size());
-  KI_ALLOC(lf.d_tasks, SweepTask, ncomp);
-  for (int t = 0; t < ncomp; t++) {
-    const Box& b = tree.boxes[boxes[t]];
-    const BoxDev& bd = boxdev_[boxes[t]];
-    st[t] = SweepTask{b.rank, static_cast<int>(b.redundant.size()), lf.d_skel + sk_off[t],
-                      lf.d_red + rd_off[t], bd.T, bd.L, bd.U, bd.X, bd.piv};
-  }
-  KI_UPLOAD(lf.d_skel, sk, ustream_);
-  KI_UPLOAD(lf.d_red, rd, ustream_);
-  KI_UPLOAD(lf.d_tasks, st, ustream_);
+  lf.boxes = boxes;
+  // one staging block and one copy: [tasks | skeleton | redundant dofs]
+  const size_t o_sk = sizeof(SweepTask) * ncomp, o_rd = o_sk + sizeof(int) * sk_off[ncomp];
+  const size_t b_pack = o_rd + sizeof(int) * rd_off[ncomp];
+  char *d_pack, *st = static_cast<char*>(stage_.alloc(b_pack));
+  if (!st) return fail("pinned staging allocation failed");
+  KI_ALLOC(d_pack, char, b_pack);
+  lf.d_tasks = reinterpret_cast<SweepTask*>(d_pack);
+  lf.d_skel = reinterpret_cast<int*>(d_pack + o_sk);
+  lf.d_red = reinterpret_cast<int*>(d_pack + o_rd);
+  lf.h_tasks.resize(ncomp);
+  parallel_for(ncomp, 32, [&](int a, int e) {
+    for (int t = a; t < e; t++) {
+      const Box& b = tree.boxes[boxes[t]];
+      const BoxDev& bd = boxdev_[boxes[t]];
+      std::copy(b.skel.begin(), b.skel.end(), reinterpret_cast<int*>(st + o_sk) + sk_off[t]);
+      std::copy(b.redundant.begin(), b.redundant.end(),
+                reinterpret_cast<int*>(st + o_rd) + rd_off[t]);
+      lf.h_tasks[t] = SweepTask{b.rank, static_cast<int>(b.redundant.size()),
+                                lf.d_skel + sk_off[t], lf.d_red + rd_off[t], bd.T, bd.L, bd.U,
+                                bd.X, bd.piv};
+    }
+  });
+  std::memcpy(st, lf.h_tasks.data(), sizeof(SweepTask) * ncomp);
+  KI_CUDA(cudaMemcpyAsync(d_pack, st, b_pack, cudaMemcpyHostToDevice, ustream_));
   KI_CUDA(cudaEventRecord(ev_up_, ustream_));
   KI_CUDA(cudaStreamWaitEvent(s, ev_up_, 0));
-  lf.h_tasks = st;
   lf.ntasks = ncomp;
-  lf.nred = static_cast<int>(rd.size());
+  lf.nred = rd_off[ncomp];
   lf.cap = cap;
   lf.kr = kr;
   return 0;
@@ -1576,14 +1591,11 @@ int Solver::update(int n_points, const double* points, const double* normals,
   cudaEvent_t ev0;
   int rc = begin_factor(&ev0);
   if (rc) return rc;
-  const std::vector<double> old_pts = pts_;
+  const HostArray old_pts = pts_;
   const int n_old = n_points_;
   n_points_ = n_points;
   n_dofs_ = n_points * sd_;
-  pts_.assign(points, points + 2 * static_cast<size_t>(n_points));
-  nrm_.assign(normals, normals + 2 * static_cast<size_t>(n_points));
-  curv_.assign(curvatures, curvatures + n_points);
-  wts_.assign(weights, weights + n_points);
+  set_geometry(points, normals, curvatures, weights);
   holes_.clear();
   if (n_holes > 0) holes_.assign(holes, holes + 4 * static_cast<size_t>(n_holes));
   tree.perturb(old_pts.data(), n_old, pts_.data(), n_points_);
@@ -1657,32 +1669,42 @@ Solver* Solver::copy(cudaStream_t stream, int* rc) {
 
 int Solver::build_all_compressed() {
   // concatenated sweep tasks of every compressed box for the diagonal solves
-  std::vector<SweepTask> all;
-  int cap = 0;
-  for (LevelFactors& lf : levels_) {
+  int cap = 0, total = 0, r_max = 0;
+  for (const LevelFactors& lf : levels_) {
     if (!lf.ntasks) continue;
-    all.insert(all.end(), lf.h_tasks.begin(), lf.h_tasks.end());
+    total += lf.ntasks;
     cap = std::max(cap, lf.cap);
+    for (const SweepTask& t : lf.h_tasks) r_max = std::max(r_max, t.r);
   }
+  all_compressed_.ntasks = total;
+  all_compressed_.cap = cap;
+  all_compressed_.nbig = all_compressed_.kr = 0;
+  KI_ALLOC(all_compressed_.d_tasks, SweepTask, total);
+  if (!total) return 0;
   // the boxes (disjoint redundant dofs, any order) by descending r: the
   // large ones first, then those whose X^{-1} a single-right-hand-side
-  // diagonal solve stages in shared memory (a launch of their own)
-  std::stable_sort(all.begin(), all.end(),
-                   [](const SweepTask& a, const SweepTask& b) { return a.r > b.r; });
-  int nbig = 0, kr = 0;
-  for (const SweepTask& t : all) {
-    if (static_cast<long long>(t.r) * t.r > kDiagStageMaxR * kDiagStageMaxR) {
-      nbig++;
-    } else {
-      kr = std::max(kr, t.r * t.r);
+  // diagonal solve stages in shared memory (a launch of their own).  Placed
+  // by counting, straight into the copy's staging.
+  std::vector<int> start(r_max + 2, 0);
+  for (const LevelFactors& lf : levels_)
+    if (lf.ntasks)
+      for (const SweepTask& t : lf.h_tasks) start[r_max - t.r + 1]++;
+  for (int i = 0; i <= r_max; i++) start[i + 1] += start[i];
+  SweepTask* st = static_cast<SweepTask*>(stage_.alloc(sizeof(SweepTask) * total));
+  if (!st) return fail("pinned staging allocation failed");
+  for (const LevelFactors& lf : levels_) {
+    if (!lf.ntasks) continue;
+    for (const SweepTask& t : lf.h_tasks) {
+      st[start[r_max - t.r]++] = t;
+      if (static_cast<long long>(t.r) * t.r > kDiagStageMaxR * kDiagStageMaxR) {
+        all_compressed_.nbig++;
+      } else {
+        all_compressed_.kr = std::max(all_compressed_.kr, t.r * t.r);
+      }
     }
   }
-  all_compressed_.ntasks = static_cast<int>(all.size());
-  all_compressed_.cap = cap;
-  all_compressed_.nbig = nbig;
-  all_compressed_.kr = kr;
-  KI_ALLOC(all_compressed_.d_tasks, SweepTask, all.size());
-  KI_UPLOAD(all_compressed_.d_tasks, all, stream_);
+  KI_CUDA(cudaMemcpyAsync(all_compressed_.d_tasks, st, sizeof(SweepTask) * total,
+                          cudaMemcpyHostToDevice, stream_));
   return 0;
 }
 
@@ -1712,63 +1734,55 @@ int Solver::factor_top_forest() {
   // the accumulated updates of the root's children, one LU per tree.
   if (build_all_compressed()) return -2;
   const int P = static_cast<int>(tree.roots.size());
-  std::vector<int> dofs, bid, bpos;
-  std::vector<UpdBlock> tab;
-  std::vector<size_t> d_off(P), b_off(P), t_off(P), a_off(P), p_off(P);
-  size_t a_total = 0, p_total = 0;
+  std::vector<std::vector<BoxBlock>> blk(P);
+  parallel_for(P, 1, [&](int a, int e) {
+    for (int p = a; p < e; p++) child_blocks(tree.roots[p], 0, &blk[p]);
+  }, 16);
+  std::vector<size_t> d_off(P), t_off(P), a_off(P);
+  size_t a_total = 0, p_total = 0, t_total = 0;
   forest_nmax_ = 0;
   for (int p = 0; p < P; p++) {
     const Box& root = tree.boxes[tree.roots[p]];
     const int n = static_cast<int>(root.active.size());
-    std::vector<BoxBlock> blocks;
-    if (!root.leaf) {
-      int off = 0;
-      for (int q = 0; q < 4; q++) {
-        const int ch = root.child[q];
-        for (const BoxBlock& x : blocks_of(ch)) blocks.push_back(BoxBlock{x.acc, x.size, x.pos + off});
-        const Box& cb = tree.boxes[ch];
-        off += static_cast<int>(cb.compressed ? cb.skel.size() : cb.active.size());
-      }
-    }
-    std::vector<int> tb, tp;
-    std::vector<UpdBlock> tt;
-    build_block_map(blocks, n, &tb, &tp, &tt);
-    d_off[p] = dofs.size();
-    b_off[p] = bid.size();
-    t_off[p] = tab.size();
+    d_off[p] = p_total;
+    t_off[p] = t_total;
     a_off[p] = a_total;
-    p_off[p] = p_total;
-    dofs.insert(dofs.end(), root.active.begin(), root.active.end());
-    bid.insert(bid.end(), tb.begin(), tb.end());
-    bpos.insert(bpos.end(), tp.begin(), tp.end());
-    tab.insert(tab.end(), tt.begin(), tt.end());
+    t_total += blk[p].size();
     a_total += static_cast<size_t>(n) * n;
     p_total += n;
     forest_nmax_ = std::max(forest_nmax_, n);
   }
   if (static_cast<size_t>(forest_nmax_) * sizeof(double) > 200 * 1024)
     return fail("a forest tree's top skeleton is too large for the batched top solve");
-  int *d_dofs, *d_bid, *d_bpos, *d_piv;
-  UpdBlock* d_tab;
+  // one staging block and one copy: [tasks | update blocks | dofs | block of
+  // each position | place in it]
+  const size_t o_tab = sizeof(TopTask) * P, o_ints = o_tab + sizeof(UpdBlock) * t_total;
+  const size_t b_pack = o_ints + sizeof(int) * 3 * p_total;
+  char *d_pack, *st = static_cast<char*>(stage_.alloc(b_pack));
+  if (!st) return fail("pinned staging allocation failed");
   double* d_a;
-  KI_ALLOC(d_dofs, int, dofs.size());
-  KI_ALLOC(d_bid, int, bid.size());
-  KI_ALLOC(d_bpos, int, bpos.size());
-  KI_ALLOC(d_tab, UpdBlock, tab.size());
+  int* d_piv;
+  KI_ALLOC(d_pack, char, b_pack);
   KI_ALLOC(d_a, double, a_total);
   KI_ALLOC(d_piv, int, p_total);
-  KI_ALLOC(d_forest_, TopTask, P);
-  std::vector<TopTask> tasks(P);
-  for (int p = 0; p < P; p++) {
-    const int n = static_cast<int>(tree.boxes[tree.roots[p]].active.size());
-    tasks[p] = TopTask{n, 0, d_dofs + d_off[p], d_bid + b_off[p], d_bpos + b_off[p],
-                       d_tab + t_off[p], d_a + a_off[p], d_piv + p_off[p]};
-  }
-  KI_UPLOAD(d_dofs, dofs, stream_);
-  KI_UPLOAD(d_bid, bid, stream_);
-  KI_UPLOAD(d_bpos, bpos, stream_);
-  KI_UPLOAD(d_tab, tab, stream_);
-  KI_UPLOAD(d_forest_, tasks, stream_);
+  d_forest_ = reinterpret_cast<TopTask*>(d_pack);
+  UpdBlock* d_tab = reinterpret_cast<UpdBlock*>(d_pack + o_tab);
+  int* d_dofs = reinterpret_cast<int*>(d_pack + o_ints);
+  int *d_bid = d_dofs + p_total, *d_bpos = d_bid + p_total;
+  parallel_for(P, 1, [&](int a, int e) {
+    int* h = reinterpret_cast<int*>(st + o_ints);
+    for (int p = a; p < e; p++) {
+      const std::vector<int>& act = tree.boxes[tree.roots[p]].active;
+      const int n = static_cast<int>(act.size());
+      std::copy(act.begin(), act.end(), h + d_off[p]);
+      fill_block_map(blk[p], n, h + p_total + d_off[p], h + 2 * p_total + d_off[p],
+                     reinterpret_cast<UpdBlock*>(st + o_tab) + t_off[p]);
+      reinterpret_cast<TopTask*>(st)[p] =
+          TopTask{n, 0, d_dofs + d_off[p], d_bid + d_off[p], d_bpos + d_off[p],
+                  d_tab + t_off[p], d_a + a_off[p], d_piv + d_off[p]};
+    }
+  }, 16);
+  KI_CUDA(cudaMemcpyAsync(d_pack, st, b_pack, cudaMemcpyHostToDevice, stream_));
   ns_ = static_cast<int>(allskel.size());
   KI_ALLOC(d_tmp_, double, 4 * static_cast<size_t>(n_dofs_) + 64);
   cudaEvent_t l0 = nullptr;
@@ -1784,21 +1798,10 @@ int Solver::factor_top() {
   KI_ALLOC(d_allskel_, int, ns_);
   KI_UPLOAD(d_allskel_, allskel, stream_);
   std::vector<BoxBlock> blocks;
-  {
-    const Box& root = tree.boxes[0];
-    if (!root.leaf) {
-      int off = 0;
-      for (int q = 0; q < 4; q++) {
-        const int ch = root.child[q];
-        for (const BoxBlock& x : blocks_of(ch)) blocks.push_back(BoxBlock{x.acc, x.size, x.pos + off});
-        const Box& cb = tree.boxes[ch];
-        off += static_cast<int>(cb.compressed ? cb.skel.size() : cb.active.size());
-      }
-    }
-  }
-  std::vector<int> bid, bpos;
-  std::vector<UpdBlock> tab;
-  build_block_map(blocks, ns_, &bid, &bpos, &tab);
+  child_blocks(0, 0, &blocks);
+  std::vector<int> bid(ns_), bpos(ns_);
+  std::vector<UpdBlock> tab(blocks.size());
+  fill_block_map(blocks, ns_, bid.data(), bpos.data(), tab.data());
   int *d_bid, *d_bpos;
   UpdBlock* d_tab;
   KI_ALLOC(d_bid, int, bid.size());

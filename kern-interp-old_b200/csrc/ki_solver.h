@@ -10,6 +10,8 @@
 
 #include <cuda_runtime.h>
 
+#include <memory>
+#include <new>
 #include <string>
 #include <utility>
 #include <vector>
@@ -103,6 +105,25 @@ struct BoxDevView {
   const int* piv;
   int k, r;
 };
+
+// Host array whose resize leaves new values uninitialised (they are filled in
+// parallel).
+template <class T>
+struct NoInit : std::allocator<T> {
+  template <class U>
+  struct rebind {
+    using other = NoInit<U>;
+  };
+  template <class U>
+  void construct(U* p) {
+    ::new (static_cast<void*>(p)) U;
+  }
+  template <class U, class... A>
+  void construct(U* p, A&&... a) {
+    ::new (static_cast<void*>(p)) U(std::forward<A>(a)...);
+  }
+};
+using HostArray = std::vector<double, NoInit<double>>;
 
 struct LevelFactors {
   int level = 0;
@@ -327,13 +348,16 @@ class Solver {
   int factor_top();
   int factor_top_forest();
   int factor_border();
-  std::vector<BoxBlock> blocks_of(int box) const;
-  void build_block_map(const std::vector<BoxBlock>& blocks, int n, std::vector<int>* bid,
-                       std::vector<int>* bpos, std::vector<UpdBlock>* tab) const;
+  void child_blocks(int box, int off, std::vector<BoxBlock>* out) const;
+  static void fill_block_map(const std::vector<BoxBlock>& blocks, int n, int* bid, int* bpos,
+                             UpdBlock* tab);
+  void set_geometry(const double* points, const double* normals, const double* curvatures,
+                    const double* weights);
 
   SolverOptions opt_;
   int sd_ = 1, n_points_ = 0, n_dofs_ = 0, nb_ = 0;
-  std::vector<double> pts_, nrm_, curv_, wts_, holes_;
+  HostArray pts_, nrm_, curv_, wts_;
+  std::vector<double> holes_;
   cudaStream_t stream_;
   // Decoupling of level l runs on dstream_ while the host prepares, and the
   // GPU runs, the interpolative decompositions of level l - 1.
