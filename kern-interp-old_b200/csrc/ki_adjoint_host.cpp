@@ -24,11 +24,11 @@ int Solver::solve_transpose_device(const double* d_b, double* d_x) {
   for (int l = L - 1; l >= 0; l--) {
     const LevelFactors& lf = levels_[l];
     if (!lf.ntasks) continue;
-    SweepParams sp{lf.d_tasks, lf.ntasks, d_x, N, 1, 0, nullptr, lf.cap};
+    SweepParams sp{lf.d_tasks, lf.ntasks, d_x, N, 1, lf.cap};
     sp.kr = lf.kr;
     KI_CUDA(launch_sweep_up(sp, true, stream_));
   }
-  SweepParams dp{all_compressed_.d_tasks, all_compressed_.ntasks, d_x, N, 1, 0, nullptr,
+  SweepParams dp{all_compressed_.d_tasks, all_compressed_.ntasks, d_x, N, 1,
                  all_compressed_.cap};
   if (diag_all(dp, true)) return -2;
   const int ns = ns_;
@@ -40,7 +40,7 @@ int Solver::solve_transpose_device(const double* d_b, double* d_x) {
   for (int l = 0; l < L; l++) {
     const LevelFactors& lf = levels_[l];
     if (!lf.ntasks) continue;
-    SweepParams sp{lf.d_tasks, lf.ntasks, d_x, N, 1, 0, nullptr, lf.cap};
+    SweepParams sp{lf.d_tasks, lf.ntasks, d_x, N, 1, lf.cap};
     sp.kr = lf.kr;
     KI_CUDA(launch_transposed_up(sp, stream_));
   }

@@ -815,14 +815,6 @@ __global__ void gather_kernel(const double* x, int ldx, const int* idx, int n, i
   out[i + static_cast<long long>(ldo) * c] = x[idx[i] + static_cast<long long>(ldx) * c];
 }
 
-__global__ void gather_rows_kernel(const double* x, int ldd, const int* idx, int n, int nrhs,
-                                   double* out, int ldo) {
-  const long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (e >= static_cast<long long>(n) * nrhs) return;
-  const int c = static_cast<int>(e % nrhs), i = static_cast<int>(e / nrhs);
-  out[i + static_cast<long long>(ldo) * c] = x[static_cast<long long>(idx[i]) * ldd + c];
-}
-
 __global__ void scatter_kernel(double* x, int ldx, const int* idx, int n, int nrhs,
                                const double* in, int ldi) {
   const long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
@@ -1592,11 +1584,11 @@ cudaError_t launch_gather(const double* x, int ldx, const int* idx, int n, int n
 // Redundant-dof index of the bordered system (skel_factorization.cpp:
 // 130-160 splits the dofs into the top level's skeletons and the rest):
 // allred = the dofs outside the ascending, repeat-free skeleton list, in
-// ascending order; red_pos[d] = d's position in allred, -1 for a skeleton.
+// ascending order.
 // A dof's position is d minus the skeletons below it (binary search), so
 // the lists are made where they are used instead of on the host.
 __global__ void red_index_kernel(const int* __restrict__ skel_sorted, int ns, int n,
-                                 int* __restrict__ allred, int* __restrict__ red_pos) {
+                                 int* __restrict__ allred) {
   const int d = blockIdx.x * blockDim.x + threadIdx.x;
   if (d >= n) return;
   int lo = 0, hi = ns;  // the first skeleton >= d
@@ -1604,29 +1596,14 @@ __global__ void red_index_kernel(const int* __restrict__ skel_sorted, int ns, in
     const int mid = (lo + hi) >> 1;
     if (skel_sorted[mid] < d) lo = mid + 1; else hi = mid;
   }
-  if (lo < ns && skel_sorted[lo] == d) {
-    red_pos[d] = -1;
-    return;
-  }
-  red_pos[d] = d - lo;
+  if (lo < ns && skel_sorted[lo] == d) return;
   allred[d - lo] = d;
 }
 
-cudaError_t launch_red_index(const int* skel_sorted, int ns, int n, int* allred, int* red_pos,
-                             cudaStream_t s) {
+cudaError_t launch_red_index(const int* skel_sorted, int ns, int n, int* allred, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   count_launches(1);
-  red_index_kernel<<<(n + 255) / 256, 256, 0, s>>>(skel_sorted, ns, n, allred, red_pos);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_gather_rows(const double* x, int ldd, const int* idx, int n, int nrhs,
-                               double* out, int ldo, cudaStream_t s) {
-  const long long tot = static_cast<long long>(n) * nrhs;
-  if (tot == 0) return cudaSuccess;
-  count_launches(1);
-  gather_rows_kernel<<<static_cast<int>((tot + 255) / 256), 256, 0, s>>>(x, ldd, idx, n, nrhs, out,
-                                                                          ldo);
+  red_index_kernel<<<(n + 255) / 256, 256, 0, s>>>(skel_sorted, ns, n, allred);
   return cudaGetLastError();
 }
 
@@ -1641,16 +1618,15 @@ cudaError_t launch_scatter(double* x, int ldx, const int* idx, int n, int nrhs,
 
 // The bordered system's row gathers in one pass (skel_factorization.cpp:
 // 146-170): U, Psi^T and X_rr^{-1} U (dof-major, nb entries a dof) at the
-// redundant dofs into Ured, Pred and dinv, U and Psi^T at the top-level
+// redundant dofs into Pred and dinv, U and Psi^T at the top-level
 // skeletons into us, ps; all outputs column-major.
 __global__ void border_gather_kernel(const double* __restrict__ modU,
                                      const double* __restrict__ modP,
                                      const double* __restrict__ modD, int nb,
                                      const int* __restrict__ allred, int nr,
                                      const int* __restrict__ allskel, int ns,
-                                     double* __restrict__ Ured, double* __restrict__ Pred,
-                                     double* __restrict__ dinv, double* __restrict__ us,
-                                     double* __restrict__ ps) {
+                                     double* __restrict__ Pred, double* __restrict__ dinv,
+                                     double* __restrict__ us, double* __restrict__ ps) {
   // the row index runs fastest: the column-major writes coalesce, and a
   // dof's nb entries, read by nb neighbouring passes, come from cache
   const long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
@@ -1659,7 +1635,6 @@ __global__ void border_gather_kernel(const double* __restrict__ modU,
   if (i < nr) {
     const long long src = static_cast<long long>(allred[i]) * nb + c;
     const long long dst = i + static_cast<long long>(nr) * c;
-    Ured[dst] = modU[src];
     dinv[dst] = modD[src];
     Pred[dst] = modP[src];
   } else {
@@ -1673,13 +1648,114 @@ __global__ void border_gather_kernel(const double* __restrict__ modU,
 
 cudaError_t launch_border_gather(const double* modU, const double* modP, const double* modD,
                                  int nb, const int* allred, int nr, const int* allskel, int ns,
-                                 double* Ured, double* Pred, double* dinv, double* us,
-                                 double* ps, cudaStream_t s) {
+                                 double* Pred, double* dinv, double* us, double* ps,
+                                 cudaStream_t s) {
   const long long tot = static_cast<long long>(nr + ns) * nb;
   if (tot == 0) return cudaSuccess;
   count_launches(1);
   border_gather_kernel<<<static_cast<int>((tot + 255) / 256), 256, 0, s>>>(
-      modU, modP, modD, nb, allred, nr, allskel, ns, Ured, Pred, dinv, us, ps);
+      modU, modP, modD, nb, allred, nr, allskel, ns, Pred, dinv, us, ps);
+  return cudaGetLastError();
+}
+
+// The border rows of a bordered solve.  Each block sums a run of rows for
+// every column: the run of x gathered into shared memory once, a warp per
+// column over it (bound by the read of Pred; runs of 256 rows give a warp
+// its eight loads at once), partial sums per block; then the sums of the
+// blocks in order, beside the gather of the skeleton rows.
+constexpr int kBorderThreads = 256, kDotThreads = 768;
+constexpr int kBorderRows = 4096;  // of a block at most (32 KB of x)
+__global__ void __launch_bounds__(kDotThreads)
+    border_dot_kernel(const double* __restrict__ Pred, int nr, int nb, int chunk,
+                      const double* __restrict__ x, const int* __restrict__ allred,
+                      double* __restrict__ part) {
+  __shared__ double xv[kBorderRows];
+  const int r0 = blockIdx.x * chunk, cnt = min(chunk, nr - r0);
+  for (int i = threadIdx.x; i < cnt; i += blockDim.x) xv[i] = x[allred[r0 + i]];
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int c = threadIdx.x >> 5; c < nb; c += blockDim.x >> 5) {
+    const double* p = Pred + static_cast<long long>(nr) * c + r0;
+    double acc[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) acc[u] = 0.0;
+    for (int i0 = 0; i0 < cnt; i0 += 256) {
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int i = i0 + 32 * u + lane;
+        if (i < cnt) acc[u] += p[i] * xv[i];
+      }
+    }
+    double s = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) part[static_cast<long long>(blockIdx.x) * nb + c] = s;
+  }
+}
+
+__global__ void border_rhs_kernel(const double* __restrict__ part, int blocks, int nb,
+                                  const double* __restrict__ x, const int* __restrict__ allskel,
+                                  int ns, const double* __restrict__ g, double* __restrict__ M) {
+  const int lane = threadIdx.x & 31;
+  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int c = w - (ns + 31) / 32;  // warps past the skeleton rows: a column each
+  if (c < 0) {
+    const int i = 32 * w + lane;
+    if (i < ns) M[i] = x[allskel[i]];
+  } else if (c < nb) {
+    double s = 0.0;
+    for (int p = lane; p < blocks; p += 32) s += part[static_cast<long long>(p) * nb + c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) M[ns + c] = (g ? g[c] : 0.0) - s;
+  }
+}
+
+int border_dot_blocks(int nr) {
+  return std::max(std::min(296, (nr + 255) / 256), (nr + kBorderRows - 1) / kBorderRows);
+}
+
+cudaError_t launch_border_rhs(const double* Pred, int nr, int nb, const double* x,
+                              const int* allred, const int* allskel, int ns, const double* g,
+                              double* part, double* M, cudaStream_t s) {
+  const int blocks = border_dot_blocks(nr);
+  count_launches(2);
+  border_dot_kernel<<<blocks, std::min(kDotThreads, 32 * nb), 0, s>>>(Pred, nr, nb, (nr + blocks - 1) / blocks, x,
+                                                      allred, part);
+  const int warps = (ns + 31) / 32 + nb;
+  border_rhs_kernel<<<(warps + 3) / 4, 128, 0, s>>>(part, blocks, nb, x, allskel, ns, g, M);
+  return cudaGetLastError();
+}
+
+// The border's part of a bordered solve's rows: X^{-1} (w - U alpha) = X^{-1}
+// w - (X^{-1} U) alpha, with X^{-1} w in x already and X^{-1} U kept by the
+// factorization, so that the diagonal blocks are read once a solve (of eight
+// holes and 65,536 dofs: this kernel and the two above 19 us, the products,
+// copies, gathers and second diagonal solve they replace about 105 us).
+__global__ void __launch_bounds__(kBorderThreads)
+    border_apply_kernel(const double* __restrict__ dinv, int nr, int nb,
+                        const int* __restrict__ allred, const int* __restrict__ allskel, int ns,
+                        const double* __restrict__ M, double* __restrict__ x,
+                        double* __restrict__ alpha) {
+  const int i = blockIdx.x * kBorderThreads + threadIdx.x;
+  const double* al = M + ns;
+  if (i < nr) {
+    double s = 0.0;
+#pragma unroll 8
+    for (int c = 0; c < nb; c++) s += dinv[i + static_cast<long long>(nr) * c] * al[c];
+    x[allred[i]] -= s;
+  } else if (i < nr + ns) {
+    x[allskel[i - nr]] = M[i - nr];
+  }
+  if (alpha && i < nb) alpha[i] = al[i];
+}
+
+cudaError_t launch_border_apply(const double* dinv, int nr, int nb, const int* allred,
+                                const int* allskel, int ns, const double* M, double* x,
+                                double* alpha, cudaStream_t s) {
+  count_launches(1);
+  border_apply_kernel<<<(std::max(nr + ns, nb) + kBorderThreads - 1) / kBorderThreads,
+                        kBorderThreads, 0, s>>>(dinv, nr, nb, allred, allskel, ns, M, x, alpha);
   return cudaGetLastError();
 }
 

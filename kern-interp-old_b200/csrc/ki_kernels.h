@@ -270,8 +270,6 @@ struct SweepParams {
   int ntasks;
   double* x;
   int ldx, nrhs;
-  int red_pos_map;      // nonzero: redundant dofs index rows of x via red_pos
-  const int* red_pos;
   int cap;              // per-box staging: max over tasks of k + r
   int ldd = 1;          // dof stride of x: entry (dof, rhs c) is x[dof ldd + c ldx]
   // nonzero: max over tasks of k r; a single right-hand side then stages the
@@ -303,16 +301,25 @@ cudaError_t launch_diag_solve_t(const SweepParams& p, cudaStream_t s);
 // out[i] = x[idx[i]] (gather) / x[idx[i]] = in[i] (scatter), nrhs columns.
 cudaError_t launch_gather(const double* x, int ldx, const int* idx, int n, int nrhs,
                           double* out, int ldo, cudaStream_t s);
-// out[i + ldo c] = x[idx[i] ldd + c]: rows of a dof-major matrix
-cudaError_t launch_gather_rows(const double* x, int ldd, const int* idx, int n, int nrhs,
-                               double* out, int ldo, cudaStream_t s);
-// Ured, Pred, dinv <- rows allred of U, Psi^T, X^{-1} U (dof-major, nb a
-// dof); us, ps <- rows allskel of U, Psi^T; outputs column-major (ld nr, ns)
+// Pred, dinv <- rows allred of Psi^T, X^{-1} U (dof-major, nb a dof); us, ps
+// <- rows allskel of U, Psi^T; outputs column-major (ld nr, ns)
 cudaError_t launch_border_gather(const double* modU, const double* modP, const double* modD,
                                  int nb,
                                  const int* allred, int nr, const int* allskel, int ns,
-                                 double* Ured, double* Pred, double* dinv, double* us,
-                                 double* ps, cudaStream_t s);
+                                 double* Pred, double* dinv, double* us, double* ps,
+                                 cudaStream_t s);
+// The border rows of a bordered solve: M[0, ns) <- x[allskel], M[ns + c] <-
+// g[c] (0 without g) - sum_i Pred(i, c) x[allred[i]]; part: border_dot_blocks(nr)
+// x nb doubles.
+int border_dot_blocks(int nr);
+cudaError_t launch_border_rhs(const double* Pred, int nr, int nb, const double* x,
+                              const int* allred, const int* allskel, int ns, const double* g,
+                              double* part, double* M, cudaStream_t s);
+// x[allred[i]] -= sum_c dinv(i, c) M[ns + c], x[allskel[i]] <- M[i], alpha
+// (if given) <- M[ns ..)
+cudaError_t launch_border_apply(const double* dinv, int nr, int nb, const int* allred,
+                                const int* allskel, int ns, const double* M, double* x,
+                                double* alpha, cudaStream_t s);
 // dst rows idx[0..n) <- the same rows of src (dof-major, nb entries a dof)
 cudaError_t launch_copy_rows(const double* src, double* dst, int nb, const int* idx, int n,
                              cudaStream_t s);
@@ -323,11 +330,9 @@ int long_gemm_tn_splits(int m, int n, int k);
 cudaError_t long_gemm_tn(int m, int n, int k, double alpha, const double* a, int lda,
                          const double* b, int ldb, double beta, double* c, int ldc,
                          double* part, cudaStream_t s);
-// allred (the n - ns dofs outside skel_sorted, ascending) and red_pos (n:
-// position in allred, -1 for a skeleton) from the ascending, repeat-free
-// skeleton dofs skel_sorted[0..ns), all below n
-cudaError_t launch_red_index(const int* skel_sorted, int ns, int n, int* allred, int* red_pos,
-                             cudaStream_t s);
+// allred (the n - ns dofs outside skel_sorted, ascending) from the ascending,
+// repeat-free skeleton dofs skel_sorted[0..ns), all below n
+cudaError_t launch_red_index(const int* skel_sorted, int ns, int n, int* allred, cudaStream_t s);
 cudaError_t launch_scatter(double* x, int ldx, const int* idx, int n, int nrhs,
                            const double* in, int ldi, cudaStream_t s);
 // C = alpha * op(A) * op(B) + beta * C, small dense FP64 (column-major).
@@ -458,8 +463,6 @@ cudaError_t launch_segment_sumsq(const double* v, const int* seg, int nseg, int 
 cudaError_t launch_add(double* x, const double* y, int n, cudaStream_t s);
 // r = b - ax
 cudaError_t launch_sub(double* r, const double* b, const double* ax, int n, cudaStream_t s);
-// y = g - y (g null: y = -y)
-cudaError_t launch_rsub(double* y, const double* g, int n, cudaStream_t s);
 
 }  // namespace kib
 

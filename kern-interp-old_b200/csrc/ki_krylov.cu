@@ -523,11 +523,6 @@ __global__ void add_kernel(double* __restrict__ x, const double* __restrict__ y,
   if (i < n) x[i] += y[i];
 }
 
-__global__ void rsub_kernel(double* __restrict__ y, const double* __restrict__ g, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] = (g ? g[i] : 0.0) - y[i];
-}
-
 __global__ void sub_kernel(double* __restrict__ r, const double* __restrict__ b,
                            const double* __restrict__ ax, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -697,13 +692,6 @@ cudaError_t launch_segment_sumsq(const double* v, const int* seg, int nseg, int 
 cudaError_t launch_add(double* x, const double* y, int n, cudaStream_t s) {
   count_launches(1);
   add_kernel<<<(n + 255) / 256, 256, 0, s>>>(x, y, n);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_rsub(double* y, const double* g, int n, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  count_launches(1);
-  rsub_kernel<<<(n + 255) / 256, 256, 0, s>>>(y, g, n);
   return cudaGetLastError();
 }
 

@@ -1242,7 +1242,7 @@ int Solver::decouple_level(PendingLevel* pl) {
     // on their own stream after the level's decoupling (in level order
     // there), off the chain of decouplings: the next level's does not read
     // them; the top level's border system waits for them
-    SweepParams sp{lf.d_tasks, lf.ntasks, d_modU_, 1, nb_, 0, nullptr, lf.cap, nb_};
+    SweepParams sp{lf.d_tasks, lf.ntasks, d_modU_, 1, nb_, lf.cap, nb_};
     SweepParams spp = sp;
     spp.x = d_modP_;
     KI_CUDA(cudaEventRecord(ev_lvl_, dstream_));
@@ -1531,8 +1531,8 @@ void Solver::drop_device_state() {
   d_top_piv_ = nullptr;
   d_top_perm_ = nullptr;
   d_top_dinv_ = nullptr;
-  d_allskel_ = d_allred_ = d_red_pos_ = nullptr;
-  d_U_ = d_Psi_ = d_Urow_ = d_Ured_ = d_Pred_ = d_tmp_ = nullptr;
+  d_allskel_ = d_allred_ = nullptr;
+  d_U_ = d_Psi_ = d_Urow_ = d_Dred_ = d_Pred_ = d_bpart_ = d_tmp_ = nullptr;
   d_modU_ = d_modP_ = d_modD_ = nullptr;
   all_compressed_ = LevelFactors{};
   levels_.clear();
@@ -1845,9 +1845,9 @@ int Solver::factor_border() {
   // skel_factorization.cpp:130-242: sweep U and Psi^T with the factors,
   // D^{-1} on the redundant rows, then the bordered Schur system S.
   const int N = n_dofs_, nb = nb_, ns = ns_;
-  // the redundant dofs (everything outside the top level's skeletons) and
-  // each dof's position among them, listed on the GPU from the sorted
-  // skeletons: no N-long host lists on the way to the top-level LU
+  // the redundant dofs (everything outside the top level's skeletons),
+  // listed on the GPU from the sorted skeletons: no N-long host lists on the
+  // way to the top-level LU
   std::vector<int> sorted = allskel;
   std::sort(sorted.begin(), sorted.end());
   for (size_t i = 0; i < sorted.size(); i++)
@@ -1859,33 +1859,31 @@ int Solver::factor_border() {
   int* d_sorted;
   KI_ALLOC(d_sorted, int, sorted.size());
   KI_ALLOC(d_allred_, int, nr);
-  KI_ALLOC(d_red_pos_, int, N);
   KI_UPLOAD(d_sorted, sorted, stream_);
-  KI_CUDA(launch_red_index(d_sorted, static_cast<int>(sorted.size()), N, d_allred_, d_red_pos_,
-                           stream_));
+  KI_CUDA(launch_red_index(d_sorted, static_cast<int>(sorted.size()), N, d_allred_, stream_));
 
   // U and Psi^T were swept up level by level with the decoupling
   double* modU = d_modU_;
   double* modP = d_modP_;
   cudaEvent_t b0 = nullptr;
   if (time_phases && timer_begin(&b0)) return -2;
-  double *dinv, *us, *ps, *corr;
-  KI_ALLOC(d_Ured_, double, static_cast<size_t>(nr) * nb);
+  double *us, *ps, *corr;
   KI_ALLOC(d_Pred_, double, static_cast<size_t>(nr) * nb);
-  KI_ALLOC(dinv, double, static_cast<size_t>(nr) * nb);
+  KI_ALLOC(d_Dred_, double, static_cast<size_t>(nr) * nb);
+  KI_ALLOC(d_bpart_, double, static_cast<size_t>(border_dot_blocks(nr)) * nb);
   KI_ALLOC(us, double, static_cast<size_t>(ns) * nb);
   KI_ALLOC(ps, double, static_cast<size_t>(ns) * nb);
   KI_ALLOC(corr, double, static_cast<size_t>(nb) * nb);
   KI_CUDA(cudaStreamWaitEvent(stream_, ev_bdr_, 0));  // U, Psi^T swept up
-  // (dinv: X_rr^{-1} U_r of every compressed box, solved level by level)
-  KI_CUDA(launch_border_gather(modU, modP, d_modD_, nb, d_allred_, nr, d_allskel_, ns, d_Ured_,
-                               d_Pred_, dinv, us, ps, stream_));
+  // (d_Dred_: X_rr^{-1} U_r of every compressed box, solved level by level)
+  KI_CUDA(launch_border_gather(modU, modP, d_modD_, nb, d_allred_, nr, d_allskel_, ns, d_Pred_,
+                               d_Dred_, us, ps, stream_));
   if (const int splits = long_gemm_tn_splits(nb, nb, nr)) {
     double* part;
     KI_ALLOC(part, double, static_cast<size_t>(splits) * nb * nb);
-    KI_CUDA(long_gemm_tn(nb, nb, nr, 1.0, d_Pred_, nr, dinv, nr, 0.0, corr, nb, part, stream_));
+    KI_CUDA(long_gemm_tn(nb, nb, nr, 1.0, d_Pred_, nr, d_Dred_, nr, 0.0, corr, nb, part, stream_));
   } else {
-    KI_CUDA(small_gemm(true, false, nb, nb, nr, 1.0, d_Pred_, nr, dinv, nr, 0.0, corr, nb,
+    KI_CUDA(small_gemm(true, false, nb, nb, nr, 1.0, d_Pred_, nr, d_Dred_, nr, 0.0, corr, nb,
                        stream_));
   }
   KI_CUDA(launch_fill_border(d_top_, ns + nb, ns, nb, us, ps, corr, stream_));
@@ -1907,18 +1905,18 @@ int Solver::solve_device(const double* d_b, double* d_mu, double* d_alpha, const
   for (int l = L - 1; l >= 0; l--) {
     const LevelFactors& lf = levels_[l];
     if (!lf.ntasks) continue;
-    SweepParams sp{lf.d_tasks, lf.ntasks, x, N, 1, 0, nullptr, lf.cap};
+    SweepParams sp{lf.d_tasks, lf.ntasks, x, N, 1, lf.cap};
     sp.kr = lf.kr;
     KI_CUDA(launch_sweep_up(sp, false, stream_));
   }
   const int ns = ns_, nb = nb_;
   if (d_forest_) {
-    SweepParams dp{all_compressed_.d_tasks, all_compressed_.ntasks, x, N, 1, 0, nullptr,
+    SweepParams dp{all_compressed_.d_tasks, all_compressed_.ntasks, x, N, 1,
                    all_compressed_.cap};
     if (diag_all(dp, false)) return -2;
     KI_CUDA(launch_forest_top_solve(d_forest_, n_trees(), forest_nmax_, x, stream_));
   } else if (nb == 0) {
-    SweepParams dp{all_compressed_.d_tasks, all_compressed_.ntasks, x, N, 1, 0, nullptr,
+    SweepParams dp{all_compressed_.d_tasks, all_compressed_.ntasks, x, N, 1,
                    all_compressed_.cap};
     if (diag_all(dp, false)) return -2;
     if (ns > 0) {
@@ -1928,43 +1926,22 @@ int Solver::solve_device(const double* d_b, double* d_mu, double* d_alpha, const
       KI_CUDA(launch_scatter(x, N, d_allskel_, ns, 1, d_tmp_, ns, stream_));
     }
   } else {
-    const int nr = n_red_;
-    double* w = d_tmp_;
-    double* dw = w + nr;
-    double* M = dw + nr;
-    KI_CUDA(launch_gather(x, N, d_allred_, nr, 1, w, nr, stream_));
-    KI_CUDA(launch_gather(x, N, d_allskel_, ns, 1, M, ns, stream_));
-    KI_CUDA(cudaMemcpyAsync(dw, w, sizeof(double) * nr, cudaMemcpyDeviceToDevice, stream_));
-    SweepParams dp{all_compressed_.d_tasks, all_compressed_.ntasks, dw, nr, 1, 1, d_red_pos_,
-                   all_compressed_.cap};
+    // x_r <- X^{-1} x_r; the bordered system's right-hand side [x_s; g -
+    // Psi~_r x_r] and solution M = [mu_s; alpha]; x_r -= (X^{-1} U~_r) alpha
+    double* M = d_tmp_;
+    SweepParams dp{all_compressed_.d_tasks, all_compressed_.ntasks, x, N, 1, all_compressed_.cap};
     if (diag_all(dp, false)) return -2;
-    // border rows of the reduced system: g - Psi~_r D^-1 w_r (the nb dot
-    // products in one pass over the rows, partials behind M)
-    if (nb <= kMaxKrylov) {
-      KI_CUDA(launch_multi_dot(d_Pred_, nr, nb, dw, nr, M + ns + nb, M + ns, stream_));
-      KI_CUDA(launch_rsub(M + ns, d_g, nb, stream_));
-    } else {
-      if (d_g)
-        KI_CUDA(cudaMemcpyAsync(M + ns, d_g, sizeof(double) * nb, cudaMemcpyDeviceToDevice,
-                                stream_));
-      KI_CUDA(small_gemm(true, false, nb, 1, nr, -1.0, d_Pred_, nr, dw, nr, d_g ? 1.0 : 0.0,
-                         M + ns, nb, stream_));
-    }
+    KI_CUDA(launch_border_rhs(d_Pred_, n_red_, nb, x, d_allred_, d_allskel_, ns, d_g, d_bpart_, M,
+                              stream_));
     KI_CUDA(dense_lu_solve(d_top_, ns + nb, ns + nb, d_top_piv_, M, 1, ns + nb, stream_,
                            d_top_perm_, d_top_dinv_));
-    if (d_alpha)
-      KI_CUDA(cudaMemcpyAsync(d_alpha, M + ns, sizeof(double) * nb, cudaMemcpyDeviceToDevice,
-                              stream_));
-    KI_CUDA(small_gemm(false, false, nr, 1, nb, -1.0, d_Ured_, nr, M + ns, nb, 1.0, w, nr, stream_));
-    dp.x = w;
-    if (diag_all(dp, false)) return -2;
-    KI_CUDA(launch_scatter(x, N, d_allred_, nr, 1, w, nr, stream_));
-    KI_CUDA(launch_scatter(x, N, d_allskel_, ns, 1, M, ns, stream_));
+    KI_CUDA(launch_border_apply(d_Dred_, n_red_, nb, d_allred_, d_allskel_, ns, M, x, d_alpha,
+                                stream_));
   }
   for (int l = 0; l < L; l++) {
     const LevelFactors& lf = levels_[l];
     if (!lf.ntasks) continue;
-    SweepParams sp{lf.d_tasks, lf.ntasks, x, N, 1, 0, nullptr, lf.cap};
+    SweepParams sp{lf.d_tasks, lf.ntasks, x, N, 1, lf.cap};
     sp.kr = lf.kr;
     KI_CUDA(launch_sweep_down(sp, stream_));
   }

@@ -425,7 +425,6 @@ class Solver {
   double* d_top_dinv_ = nullptr;  // its inverted 16 x 16 diagonal blocks (or nullptr)
   int* d_allskel_ = nullptr;
   int* d_allred_ = nullptr;
-  int* d_red_pos_ = nullptr;
   double* d_U_ = nullptr;     // N x nb
   double* d_Psi_ = nullptr;   // nb x N
   double* d_Urow_ = nullptr;  // U dof-major (N x nb, row i contiguous)
@@ -434,7 +433,8 @@ class Solver {
   // X_rr^{-1} U at every compressed box's redundant rows (dof-major), filled
   // level by level on the border stream
   double* d_modD_ = nullptr;
-  double* d_Ured_ = nullptr;  // modified U rows of allred (|red| x nb)
+  double* d_Dred_ = nullptr;  // X_rr^{-1} times the modified U rows of allred (|red| x nb)
+  double* d_bpart_ = nullptr;  // partial sums of launch_border_rhs
   double* d_Pred_ = nullptr;  // modified Psi^T rows of allred (|red| x nb)
   double* d_tmp_ = nullptr;   // solve scratch
   // refinement workspace: Krylov basis V, preconditioned basis Z, vectors,

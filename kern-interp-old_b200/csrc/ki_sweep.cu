@@ -10,10 +10,14 @@
 //   down:  x[r] -= U x[s];    x[s] -= T x[r]
 // Staged vectors are stored dof-major (row * nc + rhs) so the threads that
 // share a matrix entry read consecutive shared-memory words.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "ki_blockla.cuh"
 #include "ki_kernels.h"
+
+namespace cg = cooperative_groups;
 
 namespace kib {
 
@@ -41,10 +45,6 @@ __device__ __forceinline__ void cp_async_wait_all() {
 }
 __device__ __forceinline__ void stage_async(double* dst, const double* src, int cnt) {
   for (int e = threadIdx.x; e < cnt; e += blockDim.x) cp_async8(dst + e, src + e);
-}
-
-__device__ __forceinline__ int row_of(const SweepParams& P, int dof) {
-  return P.red_pos_map ? P.red_pos[dof] : dof;
 }
 
 // out[i, c] -= sum_l M(i, l) * in[l, c] with M(i, l) = A[i * si + l * sl].
@@ -108,35 +108,55 @@ __device__ __forceinline__ void apply_sub_multi(double* out, const double* in, i
   }
 }
 
-// One right-hand side on a wide CTA (a level of a few large boxes, the
-// factors read from global memory): where the inner index is contiguous
-// (sl = 1) a warp per output row, lanes over the inner index (coalesced,
-// eight loads in flight per lane per pass); otherwise threads over the
-// contiguous rows with the inner index cut into segments, partial sums
-// through shared memory (part: segments x rows doubles) added in segment
-// order.  Ends with a barrier.
+// A level of a few large boxes, one right-hand side, the factors read from
+// global memory: each box is swept by a cluster of kWideCluster CTAs, which
+// deal the rows of a product among themselves (a single SM's loads, and not
+// the HBM, would bound a box on one CTA).  The rows [r0, r0 + cnt) of CTA g,
+// whole 32-byte sectors:
 constexpr int kWideThreads = 512;
+constexpr int kWideCluster = 8;
+__device__ __forceinline__ void wide_rows(int rows, int g, int* r0, int* cnt) {
+  const int c = ((rows + kWideCluster - 1) / kWideCluster + 3) & ~3;
+  *r0 = min(rows, g * c);
+  *cnt = min(rows - *r0, c);
+}
+
+// out[i] -= sum_l A[i si + l sl] in[l] for i < rows on such a CTA: where the
+// inner index is contiguous (sl = 1) a warp per four output rows, lanes over
+// the inner index (coalesced, sixteen loads in flight per lane); otherwise
+// threads over the contiguous rows with the inner index cut into segments,
+// partial sums through shared memory (part: segments x rows doubles) added
+// in segment order.  Ends with a barrier.
 __device__ __forceinline__ void apply_sub_wide(double* out, const double* in, int rows, int inner,
                                                const double* A, long long si, long long sl,
                                                double* part) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (sl == 1) {
-    for (int i = warp; i < rows; i += nw) {
-      const double* a = A + si * i;
-      double acc[8];
+    for (int i0 = 4 * warp; i0 < rows; i0 += 4 * nw) {
+      const double* a[4];
+      double acc[4];
 #pragma unroll
-      for (int u = 0; u < 8; u++) acc[u] = 0.0;
-      for (int l0 = 0; l0 < inner; l0 += 256) {
+      for (int q = 0; q < 4; q++) {
+        a[q] = A + si * min(i0 + q, rows - 1);
+        acc[q] = 0.0;
+      }
+      for (int l0 = 0; l0 < inner; l0 += 128) {
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
+        for (int u = 0; u < 4; u++) {
           const int l = l0 + 32 * u + lane;
-          if (l < inner) acc[u] += a[l] * in[l];
+          if (l < inner) {
+            const double v = in[l];
+#pragma unroll
+            for (int q = 0; q < 4; q++) acc[q] += a[q][l] * v;
+          }
         }
       }
-      double s = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) out[i] -= s;
+      for (int q = 0; q < 4; q++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+        if (lane == 0 && i0 + q < rows) out[i0 + q] -= acc[q];
+      }
     }
     __syncthreads();
     return;
@@ -172,11 +192,8 @@ __device__ __forceinline__ void apply_sub_wide(double* out, const double* in, in
 }
 
 __device__ __forceinline__ void apply_any(double* out, const double* in, int rows, int inner,
-                                          int nc, const double* A, long long si, long long sl,
-                                          double* part = nullptr) {
-  if (part) {
-    apply_sub_wide(out, in, rows, inner, A, si, sl, part);
-  } else if (nc == 1) {
+                                          int nc, const double* A, long long si, long long sl) {
+  if (nc == 1) {
     apply_sub(out, in, rows, inner, nc, A, si, sl);
   } else {
     apply_sub_multi(out, in, rows, inner, nc, A, si, sl);
@@ -184,8 +201,7 @@ __device__ __forceinline__ void apply_any(double* out, const double* in, int row
 }
 
 template <int MODE>  // 0 up (L), 1 up (U^T), 2 down, 3 transposed up (L^T, T)
-__device__ __forceinline__ void sweep_body(const SweepParams& P, int chunk, double* sm,
-                                           bool wide = false) {
+__device__ __forceinline__ void sweep_body(const SweepParams& P, int chunk, double* sm) {
   const SweepTask tk = P.tasks[blockIdx.x];
   const int k = tk.k, r = tk.r;
   const int* S = tk.skel;
@@ -201,8 +217,6 @@ __device__ __forceinline__ void sweep_body(const SweepParams& P, int chunk, doub
     F1 = f1;
     F2 = f1 + P.kr;
   }
-  // wide CTA, one right-hand side: partial-sum scratch after the vector
-  double* part = wide && chunk == 1 ? sm + P.cap : nullptr;
   for (int c0 = 0; c0 < P.nrhs; c0 += chunk) {
     const int nc = min(chunk, P.nrhs - c0);
     double* xs = sm;
@@ -219,27 +233,27 @@ __device__ __forceinline__ void sweep_body(const SweepParams& P, int chunk, doub
     __syncthreads();
     if (MODE <= 1) {
       // xr -= T^T xs : (T^T)(j, l) = T[l + k j]
-      apply_any(xr, xs, r, k, nc, F1, k, 1, part);
+      apply_any(xr, xs, r, k, nc, F1, k, 1);
       __syncthreads();
       if (MODE == 0) {
         // xs -= L xr : L(i, j) = L[i + k j]
-        apply_any(xs, xr, k, r, nc, F2, 1, k, part);
+        apply_any(xs, xr, k, r, nc, F2, 1, k);
       } else {
         // xs -= U^T xr : (U^T)(i, j) = U[j + r i]
-        apply_any(xs, xr, k, r, nc, F2, r, 1, part);
+        apply_any(xs, xr, k, r, nc, F2, r, 1);
       }
     } else if (MODE == 2) {
       // xr -= U xs : U(j, l) = U[j + r l]
-      apply_any(xr, xs, r, k, nc, F1, 1, r, part);
+      apply_any(xr, xs, r, k, nc, F1, 1, r);
       __syncthreads();
       // xs -= T xr : T(i, j) = T[i + k j]
-      apply_any(xs, xr, k, r, nc, F2, 1, k, part);
+      apply_any(xs, xr, k, r, nc, F2, 1, k);
     } else {
       // xr -= L^T xs : (L^T)(j, l) = L[l + k j]
-      apply_any(xr, xs, r, k, nc, F1, k, 1, part);
+      apply_any(xr, xs, r, k, nc, F1, k, 1);
       __syncthreads();
       // xs -= T xr
-      apply_any(xs, xr, k, r, nc, F2, 1, k, part);
+      apply_any(xs, xr, k, r, nc, F2, 1, k);
     }
     __syncthreads();
     for (int t = threadIdx.x; t < k * nc; t += blockDim.x) {
@@ -266,17 +280,21 @@ __device__ __forceinline__ void wait_prior_grid() {
 
 template <typename... KArgs, typename... Args>
 cudaError_t launch_chained(void (*kernel)(KArgs...), int blocks, int threads, size_t smem,
-                           cudaStream_t s, Args... args) {
+                           cudaStream_t s, int cluster, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -288,13 +306,52 @@ __global__ void __launch_bounds__(kSweepThreads) sweep_kernel(SweepParams P, int
   sweep_body<MODE>(P, chunk, sm);
 }
 
-// A level of a few large boxes, one right-hand side, factors not staged:
-// 512 threads per box (see apply_sub_wide).
+// A level of a few large boxes, one right-hand side, factors not staged: a
+// cluster per box (see wide_rows).  Every CTA gathers the whole vector,
+// forms its rows of the first product, hands them to the others and forms
+// its rows of the second.  A 65,536-dof Stokes problem's four boxes of level
+// 1: 40 us -> 12 us a sweep, the sixteen of level 2: 22 us -> 11 us (one CTA
+// per box before).
 template <int MODE>
 __global__ void __launch_bounds__(kWideThreads) sweep_wide_kernel(SweepParams P) {
   wait_prior_grid();
   extern __shared__ double sm[];
-  sweep_body<MODE>(P, 1, sm, true);
+  const cg::cluster_group cl = cg::this_cluster();
+  const int g = blockIdx.x % kWideCluster;
+  const SweepTask tk = P.tasks[blockIdx.x / kWideCluster];
+  const int k = tk.k, r = tk.r;
+  double* xs = sm;
+  double* xr = sm + k;
+  double* part = sm + P.cap;
+  for (int i = threadIdx.x; i < k; i += kWideThreads)
+    xs[i] = P.x[static_cast<long long>(tk.skel[i]) * P.ldd];
+  for (int j = threadIdx.x; j < r; j += kWideThreads)
+    xr[j] = P.x[static_cast<long long>(tk.red[j]) * P.ldd];
+  cl.sync();  // every CTA of the box has its copy
+  int r0, nr, s0, ns;
+  wide_rows(r, g, &r0, &nr);
+  wide_rows(k, g, &s0, &ns);
+  if (MODE == 2) {
+    apply_sub_wide(xr + r0, xs, nr, k, tk.U + r0, 1, r, part);
+  } else {
+    apply_sub_wide(xr + r0, xs, nr, k, (MODE == 3 ? tk.L : tk.T) + static_cast<long long>(k) * r0,
+                   k, 1, part);
+  }
+  for (int gg = threadIdx.x >> 5; gg < kWideCluster; gg += kWideThreads / 32)
+    if (gg != g) {
+      double* dst = cl.map_shared_rank(xr + r0, gg);
+      for (int e = threadIdx.x & 31; e < nr; e += 32) dst[e] = xr[r0 + e];
+    }
+  cl.sync();
+  if (MODE == 1) {
+    apply_sub_wide(xs + s0, xr, ns, r, tk.U + static_cast<long long>(r) * s0, r, 1, part);
+  } else {
+    apply_sub_wide(xs + s0, xr, ns, r, (MODE == 0 ? tk.L : tk.T) + s0, 1, k, part);
+  }
+  for (int i = threadIdx.x; i < ns; i += kWideThreads)
+    P.x[static_cast<long long>(tk.skel[s0 + i]) * P.ldd] = xs[s0 + i];
+  for (int j = threadIdx.x; j < nr; j += kWideThreads)
+    P.x[static_cast<long long>(tk.red[r0 + j]) * P.ldd] = xr[r0 + j];
 }
 
 // The two up sweeps of the hole border (U with L, Psi^T with U^T) of one
@@ -335,7 +392,7 @@ __global__ void __launch_bounds__(kDiagThreads) diag_inv_kernel(SweepParams P, i
     double* ys = sm + static_cast<long long>(r) * nc;
     for (int t = threadIdx.x; t < r * nc; t += kDiagThreads) {
       const int j = t / nc, c = t - j * nc;
-      xs[t] = P.x[static_cast<long long>(row_of(P, R[j])) * P.ldd + static_cast<long long>(P.ldx) * (c0 + c)];
+      xs[t] = P.x[static_cast<long long>(R[j]) * P.ldd + static_cast<long long>(P.ldx) * (c0 + c)];
     }
     if (staged) cp_async_wait_all();
     __syncthreads();
@@ -393,7 +450,7 @@ __global__ void __launch_bounds__(kDiagThreads) diag_inv_kernel(SweepParams P, i
     __syncthreads();
     for (int t = threadIdx.x; t < r * nc; t += kDiagThreads) {
       const int j = t / nc, c = t - j * nc;
-      P.x[static_cast<long long>(row_of(P, R[j])) * P.ldd + static_cast<long long>(P.ldx) * (c0 + c)] = ys[t];
+      P.x[static_cast<long long>(R[j]) * P.ldd + static_cast<long long>(P.ldx) * (c0 + c)] = ys[t];
     }
     __syncthreads();
   }
@@ -424,13 +481,14 @@ cudaError_t launch_mode(const SweepParams& p0, cudaStream_t s) {
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(wsmem));
     if (e != cudaSuccess) return e;
-    return launch_chained(sweep_wide_kernel<MODE>, p.ntasks, kWideThreads, wsmem, s, p);
+    return launch_chained(sweep_wide_kernel<MODE>, kWideCluster * p.ntasks, kWideThreads, wsmem, s,
+                          kWideCluster, p);
   }
   cudaError_t e = raise_func_attr(reinterpret_cast<const void*>(&sweep_kernel<MODE>),
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem));
   if (e != cudaSuccess) return e;
-  return launch_chained(sweep_kernel<MODE>, p.ntasks, kSweepThreads, smem, s, p, nc);
+  return launch_chained(sweep_kernel<MODE>, p.ntasks, kSweepThreads, smem, s, 1, p, nc);
 }
 
 }  // namespace
@@ -467,31 +525,33 @@ cudaError_t launch_transposed_up(const SweepParams& p, cudaStream_t s) {
 }
 
 namespace {
-// The diagonal step of a few large boxes, one right-hand side: 512 threads
-// per box, x_r <- X^{-1} x_r through apply_sub_wide (ys = 0 - X^{-1} xs,
-// stored negated).
+// The diagonal step of a few large boxes, one right-hand side: a cluster per
+// box, x_r <- X^{-1} x_r by rows (ys = 0 - X^{-1} xs, stored negated): one
+// box of that problem 34 us -> 11 us.
 template <bool TRANS>
 __global__ void __launch_bounds__(kWideThreads) diag_wide_kernel(SweepParams P) {
   wait_prior_grid();
   extern __shared__ double sm[];
-  const SweepTask tk = P.tasks[blockIdx.x];
+  const int g = blockIdx.x % kWideCluster;
+  const SweepTask tk = P.tasks[blockIdx.x / kWideCluster];
   const int r = tk.r;
-  const int* R = tk.red;
   double* xs = sm;
   double* ys = sm + P.cap;
   double* part = ys + P.cap;
-  for (int j = threadIdx.x; j < r; j += blockDim.x) {
-    xs[j] = P.x[static_cast<long long>(row_of(P, R[j])) * P.ldd];
+  for (int j = threadIdx.x; j < r; j += kWideThreads) {
+    xs[j] = P.x[static_cast<long long>(tk.red[j]) * P.ldd];
     ys[j] = 0.0;
   }
-  __syncthreads();
-  if (TRANS) {
-    apply_sub_wide(ys, xs, r, r, tk.X, r, 1, part);  // X^{-T}(i, j) = X[j + r i]
-  } else {
-    apply_sub_wide(ys, xs, r, r, tk.X, 1, r, part);  // X^{-1}(i, j) = X[i + r j]
+  cg::this_cluster().sync();  // every CTA of the box has its copy
+  int r0, nr;
+  wide_rows(r, g, &r0, &nr);
+  if (TRANS) {  // X^{-T}(i, j) = X[j + r i]
+    apply_sub_wide(ys, xs, nr, r, tk.X + static_cast<long long>(r) * r0, r, 1, part);
+  } else {  // X^{-1}(i, j) = X[i + r j]
+    apply_sub_wide(ys, xs, nr, r, tk.X + r0, 1, r, part);
   }
-  for (int j = threadIdx.x; j < r; j += blockDim.x)
-    P.x[static_cast<long long>(row_of(P, R[j])) * P.ldd] = -ys[j];
+  for (int j = threadIdx.x; j < nr; j += kWideThreads)
+    P.x[static_cast<long long>(tk.red[r0 + j]) * P.ldd] = -ys[j];
 }
 
 template <bool TRANS>
@@ -512,14 +572,15 @@ cudaError_t launch_diag(const SweepParams& p0, cudaStream_t s) {
                                     static_cast<int>(wsmem));
     if (e != cudaSuccess) return e;
     count_launches(1);
-    return launch_chained(diag_wide_kernel<TRANS>, p.ntasks, kWideThreads, wsmem, s, p);
+    return launch_chained(diag_wide_kernel<TRANS>, kWideCluster * p.ntasks, kWideThreads, wsmem, s,
+                          kWideCluster, p);
   }
   cudaError_t e = raise_func_attr(reinterpret_cast<const void*>(&diag_inv_kernel<TRANS>),
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   count_launches(1);
-  return launch_chained(diag_inv_kernel<TRANS>, p.ntasks, kDiagThreads, smem, s, p, nc);
+  return launch_chained(diag_inv_kernel<TRANS>, p.ntasks, kDiagThreads, smem, s, 1, p, nc);
 }
 }  // namespace
 
