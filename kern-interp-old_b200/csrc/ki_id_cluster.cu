@@ -1557,6 +1557,8 @@ cudaError_t launch_id_cluster(const IdParams& p, int group, cudaStream_t s) {
     case kOnChip + 4: return launch_cluster<4, false, false>(p, s);
     case kOnChip + 8: return launch_cluster<8, false, false>(p, s);
     case kOnChip + 16: return launch_cluster<16, false, false>(p, s);
+    case kSketched + 1: return launch_cluster<1, true, false>(p, s);
+    case kSketched + 2: return launch_cluster<2, true, false>(p, s);
     case kSketched + 8: return launch_cluster<8, true, false>(p, s);
     case kSketched + 16: return launch_cluster<16, true, false>(p, s);
     case kSpilled + 8: return launch_cluster<8, false, true>(p, s);

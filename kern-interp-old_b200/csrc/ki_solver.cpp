@@ -174,9 +174,18 @@ int pick_group(int n_row, int proxy, int n, const bool* onchip_ok, int* g_slab, 
   return *g_slab;
 }
 
-// The same for an l x n sketch; 0: none.
+// The same for an l x n sketch; 0: none.  Registers of one CTA; then shared
+// memory of one or two CTAs, ahead of registers spread over more: a sketch has
+// few rows, so the exchange of a step between CTAs costs more than the slower
+// memory (212 x 196: 0.61 ms in the shared memory of two CTAs, 0.78 ms in the
+// registers of four; 168 x 152: 0.45 ms on one CTA, 0.50 ms on two.  Exact
+// boxes, of several times the rows, are the other way round: 566 x 48, 87 us
+// on one CTA, 81 us in two CTAs' registers).
 int pick_sketch_group(int l, int n, const bool* onchip_ok) {
-  for (int G = 1; G <= 16; G *= 2) {
+  if (const int t = onchip_ok[1] ? id_tile(l, n, 1) : -1; t >= 0) return kTile + 100 * t + 1;
+  for (int G = 1; G <= 2; G *= 2)
+    if (onchip_ok[G] && id_resident_columns(l, n, G) >= n) return kSketched + G;
+  for (int G = 2; G <= 16; G *= 2) {
     const int t = onchip_ok[G] ? id_tile(l, n, G) : -1;
     if (t >= 0) return kTile + 100 * t + G;
   }
