@@ -15,25 +15,6 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
-// C (m x n) = C0 - op(A) op(B) over the CTA, with op(A) m x kk, op(B) kk x n.
-// C may alias C0.  ta/tb select the transposes (A stored kk x m when ta).
-__device__ inline void cta_gemm_sub(double* C, int ldc, const double* C0, int ldc0,
-                                    const double* A, int lda, bool ta, const double* B,
-                                    int ldb, bool tb, int m, int n, int kk) {
-  for (int e = threadIdx.x; e < m * n; e += blockDim.x) {
-    const int i = e % m, j = e / m;
-    double s = 0.0;
-    for (int l = 0; l < kk; l++) {
-      const double a = ta ? A[l + static_cast<long long>(lda) * i]
-                          : A[i + static_cast<long long>(lda) * l];
-      const double b = tb ? B[j + static_cast<long long>(ldb) * l]
-                          : B[l + static_cast<long long>(ldb) * j];
-      s += a * b;
-    }
-    C[i + static_cast<long long>(ldc) * j] = C0[i + static_cast<long long>(ldc0) * j] - s;
-  }
-}
-
 // One FP64 tensor-core step (DMMA, mma.sync m8n8k4 .f64): the warp's 8 x 8
 // block C += A (8 x 4) B (4 x 8).  Fragments: lane l holds A(l / 4, l % 4),
 // B(l % 4, l / 4) and C(l / 4, 2 (l % 4) + v), v = 0, 1.
@@ -237,101 +218,6 @@ __device__ __forceinline__ void warp_argmax_bits(unsigned long long key, int idx
                                                               : 0x7fffffffu));
   *kmax = (static_cast<unsigned long long>(mhi) << 32) | mlo;
 }
-
-// Gauss-Jordan inversion of the n x n matrix a (column-major, ld; n <=
-// blockDim.x) in place, partial pivoting, one barrier per pivot step.  Row
-// i is updated by S = blockDim.x / n threads (at most 8), thread (i, s)
-// owning the columns of segment s.  Rows are never exchanged: step j
-// eliminates column j with row p_j (the largest |a(i, j)| among the rows
-// not yet pivots, the first on ties; a NaN counts as 0).  Before the step's
-// barrier the owner of a(i, j) keeps it in colj (double-buffered by step
-// parity) and each warp publishes its best candidate (key, row) in a slot;
-// after it every thread reduces the slots to the same p_j and updates its
-// segment with the arithmetic of the row-swapping form: a(i, c) -= a(i, j)
-// (a(p, c) / piv) via the reciprocal, a(i, j) <- -a(i, j) / piv, while row
-// p_j waits until the next step's barrier, when nobody reads it any more,
-// to scale itself (a(p, c) / piv, a(p, j) <- 1 / piv).  On return the
-// result B holds A^{-1}(j, q) = B(p_j, p^{-1}(q)); pivot_row[j] = p_j.
-// Returns nonzero when a pivot was 0, infinite or NaN.  Slots: 2 x 32 keys
-// and rows; colj: 2 n doubles.
-__device__ inline int cta_gj_invert_inplace(double* a, int n, int ld, int* pivot_row,
-                                            unsigned long long* slot_key, int* slot_row,
-                                            double* colj) {
-  if (n <= 0) return 0;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
-  const int S = max(1, min(static_cast<int>(blockDim.x) / n, 8));
-  const int i = t % n, sg = t / n;
-  const bool live = sg < S;
-  const int L = (n + S - 1) / S, cb = sg * L, ce = min(n, cb + L);
-  double* ar = a + i;
-  bool used = false, pending = false;
-  int jprev = 0;
-  double own_inv = 0.0;
-  int info = 0;
-  for (int j = 0; j < n; j++) {
-    const int buf = j & 1;
-    const bool owner = live && j >= cb && j < ce;
-    double aij = 0.0;
-    if (owner) {
-      aij = ar[static_cast<long long>(ld) * j];
-      if (pending) aij *= own_inv;  // (the row scales itself after the barrier)
-      colj[buf * n + i] = aij;
-    }
-    const bool cand = owner && !used;
-    double v = cand ? fabs(aij) : 0.0;
-    if (v != v) v = 0.0;
-    unsigned long long wk;
-    int wi;
-    warp_argmax_bits(cand ? static_cast<unsigned long long>(__double_as_longlong(v)) : 0ull,
-                     cand ? i : 0x7fffffff, &wk, &wi);
-    if (lane == 0) {
-      slot_key[32 * buf + warp] = wk;
-      slot_row[32 * buf + warp] = wi;
-    }
-    __syncthreads();
-    unsigned long long gk;
-    int p;
-    warp_argmax_bits(lane < nw ? slot_key[32 * buf + lane] : 0ull,
-                     lane < nw ? slot_row[32 * buf + lane] : 0x7fffffff, &gk, &p);
-    if (pending) {  // the previous step's pivot row, scaled now
-      for (int c = cb; c < ce; c++) {
-        double* e = ar + static_cast<long long>(ld) * c;
-        *e = c == jprev ? own_inv : *e * own_inv;
-      }
-      pending = false;
-    }
-    const double* ap = a + p;
-    const double piv = ap[static_cast<long long>(ld) * j];
-    if (!(fabs(piv) > 0.0) || isinf(piv)) info = 1;  // (0, NaN or infinite)
-    const double inv = 1.0 / piv;
-    if (t == 0) pivot_row[j] = p;
-    if (i == p) {
-      if (live) {
-        used = true;
-        pending = true;
-        own_inv = inv;
-        jprev = j;
-      }
-    } else if (live) {
-      const double f = colj[buf * n + i];
-#pragma unroll 4
-      for (int c = cb; c < ce; c++) {
-        double* e = ar + static_cast<long long>(ld) * c;
-        *e = c == j ? -f * inv : *e - f * (ap[static_cast<long long>(ld) * c] * inv);
-      }
-    }
-  }
-  __syncthreads();  // (every read of the last pivot row done)
-  if (pending) {
-    for (int c = cb; c < ce; c++) {
-      double* e = ar + static_cast<long long>(ld) * c;
-      *e = c == jprev ? own_inv : *e * own_inv;
-    }
-  }
-  __syncthreads();
-  return info;
-}
-
 
 // b (length n, stride inc) <- A^{-1} b for the LU above, by one warp.
 __device__ inline void warp_lu_solve(const double* lu, int n, int ld, const int* ipiv,

@@ -126,8 +126,8 @@ __device__ __forceinline__ int cta_gj_regs(double* X, int ld, int r, double* col
   for (int j = 0; j < r; j++) {
     double* cj = colj + (j & 1) * RP;
     if ((j & 7) == warp) {
-      // (comparing columns, not u: see cta_mma's callers' register arrays,
-      // which an equality on the index would turn into local memory)
+      // (comparing columns, not u: with an equality on u the compiler indexes
+      // the register array by it and puts it in local memory)
       double y[RS];
 #pragma unroll
       for (int u = 0; u < CW; u++)

@@ -472,7 +472,7 @@ cudaError_t launch_mode(const SweepParams& p0, cudaStream_t s) {
     smem += 2 * sizeof(double) * static_cast<size_t>(p.kr);
   else
     p.kr = 0;
-  if (nc == 1 && p.kr == 0 && p.ntasks <= kWideMaxBoxes) {
+  if (p.nrhs == 1 && p.kr == 0 && p.ntasks <= kWideMaxBoxes) {
     // the partial sums: segments x rows rounded to 32, at most the larger
     // of kWideThreads and the rows rounded up (a single segment)
     const size_t wsmem =
@@ -564,7 +564,7 @@ cudaError_t launch_diag(const SweepParams& p0, cudaStream_t s) {
     smem += sizeof(double) * static_cast<size_t>(p.kr);
   else
     p.kr = 0;
-  if (nc == 1 && p.kr == 0 && p.ntasks <= kWideMaxBoxes) {
+  if (p.nrhs == 1 && p.kr == 0 && p.ntasks <= kWideMaxBoxes) {
     const size_t wsmem = sizeof(double) * (2 * static_cast<size_t>(p.cap) +
                                            std::max(kWideThreads, (p.cap + 31) & ~31) + 64);
     cudaError_t e = raise_func_attr(reinterpret_cast<const void*>(&diag_wide_kernel<TRANS>),
