@@ -454,7 +454,7 @@ __host__ __device__ inline size_t oc_fixed_bytes(int m, int n, int G) {
   const int mn = m < n ? m : n;
   return sizeof(double) * (2 * static_cast<size_t>(oc_stride(m, G)) + oc_ex_doubles(n, G) + mn +
                            3 * static_cast<size_t>(n) + kOcWarps + 4) +
-         sizeof(int) * (4 * static_cast<size_t>(n) + kOcWarps + 8);
+         sizeof(int) * (5 * static_cast<size_t>(n) + kOcWarps + 8);
 }
 
 __device__ __forceinline__ double oc_warp_sum(double v) {
@@ -467,9 +467,10 @@ __device__ __forceinline__ double oc_warp_sum(double v) {
 // group takes rows r0 + 2 gl, + 2 L, ...).  Column u: x <- x - tw[u] cp (the
 // last reflector), S[u] += x c with c = ap - twp cp the new pivot column
 // below row i (rows from lo on; 0 above), and with NORM N[u] += x^2 over the
-// same rows.
+// same rows.  The result goes to dst (col, but for a column that moves).
 template <int L, int C, bool NORM>
-__device__ __forceinline__ void oc_pass(double* const (&col)[C], const double (&tw)[C],
+__device__ __forceinline__ void oc_pass(double* const (&col)[C], double* const (&dst)[C],
+                                        const double (&tw)[C],
                                         const bool (&on)[C], const double* cprev,
                                         const double* ap, double twp, int r0, int lo, int mend,
                                         int gl, double (&S)[C], double (&N)[C]) {
@@ -490,7 +491,7 @@ __device__ __forceinline__ void oc_pass(double* const (&col)[C], const double (&
       if (on[u]) {
         x[u].x = fma(-tw[u], cp.x, x[u].x);
         x[u].y = fma(-tw[u], cp.y, x[u].y);
-        *reinterpret_cast<double2*>(col[u] + r) = x[u];
+        *reinterpret_cast<double2*>(dst[u] + r) = x[u];
         S[u] = fma(x[u].x, c0, S[u]);
         S[u] = fma(x[u].y, c1, S[u]);
         if (NORM) {
@@ -639,6 +640,9 @@ __device__ __forceinline__ unsigned long long oc_cand_key(double v, int e0, bool
 // What bounds a step is its chain (warp sums, a square root, a division, two
 // barriers) and, for the larger tiles, instruction issue; few warps with
 // many columns each keep the per-warp part of that small.
+// Against the former slab in shared memory with columns dealt to the CTAs:
+// 602 x 48, 8 boxes, 167 us -> 82 us; 976 x 58, 10 boxes, 262 us -> 121 us;
+// 384 x 81, 311 us -> 181 us.
 template <int V>
 struct TileSum {  // warp sums of V values: lane holds the total of value lane / H
   static constexpr int P2 = V <= 1 ? 1 : V <= 2 ? 2 : V <= 4 ? 4 : V <= 8 ? 8 : V <= 16 ? 16 : 32;
@@ -1090,22 +1094,27 @@ __global__ void __launch_bounds__(kOcThreads, 1) id_cluster_kernel(IdParams P) {
   unsigned long long* skey = reinterpret_cast<unsigned long long*>(vn2 + n);  // kOcWarps
   double* hh = reinterpret_cast<double*>(skey + kOcWarps);  // [0] alpha (G = 1), [1] |tol R_00|
   int* sidx = reinterpret_cast<int*>(hh + 4);     // kOcWarps
-  int* si = sidx + kOcWarps;                      // [2] rank once found, [3] units
+  int* si = sidx + kOcWarps;  // [2] rank once found, [3] units, [6] next spilled column, [7] slot
   int* pos2col = si + 8;                          // n
   int* col2pos = pos2col + n;                     // n
   int* own = col2pos + n;                         // n: the trailing columns
   int* col2own = own + n;                         // n
+  int* slot = col2own + n;                        // n: a column's place (spilled ones past nres)
   // R's rows when they are spread over a cluster, then the spilled columns
   double* Rg = P.work + tk.a_off;                 // [mn][n]
   double* spill = nullptr;
   if constexpr (SPILL)
     spill = Rg + oc_rows_doubles(mn, n) + static_cast<long long>(g) * (n - nres) * ldl;
-  auto colp = [&](int j) -> double* {
+  auto place = [&](int q) -> double* {
     if constexpr (SPILL) {
-      if (j >= nres) return spill + static_cast<long long>(j - nres) * ldl;
+      if (q >= nres) return spill + static_cast<long long>(q - nres) * ldl;
     }
-    return slab + static_cast<size_t>(j) * ldl;
+    return slab + static_cast<size_t>(q) * ldl;
   };
+  // A pivot's place in shared memory is free a step later; the next spilled
+  // column moves there as that step's pass updates it, so that the passes
+  // through L2 shrink with every step (1400 x 422: 3.57 ms -> 3.39 ms).
+  auto colp = [&](int j) -> double* { return place(SPILL ? slot[j] : j); };
   auto barrier = [&]() {
     if constexpr (G > 1) {
       cg::this_cluster().sync();
@@ -1143,12 +1152,16 @@ __global__ void __launch_bounds__(kOcThreads, 1) id_cluster_kernel(IdParams P) {
 
   // ---- generation of this CTA's rows of every column
   for (int t = threadIdx.x; t < n; t += kOcThreads) {
-    pos2col[t] = col2pos[t] = own[t] = col2own[t] = t;
+    pos2col[t] = col2pos[t] = own[t] = col2own[t] = slot[t] = t;
     tws[t] = 0.0;
   }
   for (int e = threadIdx.x; e < 2 * ldl; e += kOcThreads) cb[e] = 0.0;
-  if (threadIdx.x == 0) si[2] = 0;
-  oc_generate<SK, kOcWarps>(P, tk, mg, ldl, g, G, ex, si, colp);
+  if (threadIdx.x == 0) {
+    si[2] = 0;
+    si[6] = nres;
+    si[7] = -1;
+  }
+  oc_generate<SK, kOcWarps>(P, tk, mg, ldl, g, G, ex, si, place);
   barrier();  // (every CTA done with its column records: the sums take their place)
   // ---- initial norms
   for (int t = warp; t < n; t += kOcWarps) {
@@ -1242,6 +1255,17 @@ __global__ void __launch_bounds__(kOcThreads, 1) id_cluster_kernel(IdParams P) {
     double* cnew = cb + (i & 1) * ldl;
     const double* ap = colp(p);
     const double twp = tws[p];
+    int mv = -1;  // the column that moves to the free place to
+    double* to = nullptr;
+    if constexpr (SPILL) {
+      if (si[7] >= 0) {
+        to = place(si[7]);
+        // (col2pos changes under this for the pivot and the column it trades
+        // places with, which stays at i or past it)
+        for (int j = si[6]; j < n && mv < 0; j++)
+          if (j != p && col2pos[j] >= i) mv = j;
+      }
+    }
     const int nunit = (cnt + per - 1) >> lp;
     for (int u = warp; u <= nunit; u += kOcWarps) {
       if (u == nunit) {
@@ -1276,7 +1300,7 @@ __global__ void __launch_bounds__(kOcThreads, 1) id_cluster_kernel(IdParams P) {
       auto unit_pass = [&](auto lc, auto cc) {
         constexpr int L = decltype(lc)::value, C = decltype(cc)::value;
         const int gl = lane & (L - 1), q0 = (u << lp) + lane / L * C;
-        double* col[C];
+        double *col[C], *dst[C];
         double tw[C], S[C], N[C];
         bool on[C];
 #pragma unroll
@@ -1284,12 +1308,13 @@ __global__ void __launch_bounds__(kOcThreads, 1) id_cluster_kernel(IdParams P) {
           on[v] = q0 + v < cnt;
           const int j = on[v] ? list(q0 + v) : p;
           col[v] = colp(j);
+          dst[v] = SPILL && j == mv ? to : col[v];
           tw[v] = tws[j];
         }
         if (norm) {
-          oc_pass<L, C, true>(col, tw, on, cprev, ap, twp, r0, lo, mend, gl, S, N);
+          oc_pass<L, C, true>(col, dst, tw, on, cprev, ap, twp, r0, lo, mend, gl, S, N);
         } else {
-          oc_pass<L, C, false>(col, tw, on, cprev, ap, twp, r0, lo, mend, gl, S, N);
+          oc_pass<L, C, false>(col, dst, tw, on, cprev, ap, twp, r0, lo, mend, gl, S, N);
         }
         const double s = oc_group_sum<L, C>(S, gl);
         const double nn = norm ? oc_group_sum<L, C>(N, gl) : 0.0;
@@ -1301,7 +1326,7 @@ __global__ void __launch_bounds__(kOcThreads, 1) id_cluster_kernel(IdParams P) {
           const int j = list(q0 + v);
           loc[j] = s;
           if (norm) loc[wslot + lane / L * C + v] = nn;
-          if (G > 1 && iown) loci[j] = colp(j)[iloc];
+          if (G > 1 && iown) loci[j] = (SPILL && j == mv ? to : colp(j))[iloc];
         }
       };
       if constexpr (!SK) {
@@ -1313,6 +1338,15 @@ __global__ void __launch_bounds__(kOcThreads, 1) id_cluster_kernel(IdParams P) {
       unit_pass(std::integral_constant<int, 8>{}, std::integral_constant<int, 2>{});
     }
     exchange(b, iown);
+    if constexpr (SPILL) {
+      if (threadIdx.x == kOcThreads - 1) {  // (nobody reads these before the next barrier)
+        if (mv >= 0) {
+          slot[mv] = si[7];
+          si[6] = mv + 1;
+        }
+        si[7] = slot[p] < nres ? slot[p] : -1;
+      }
+    }
 
     // ---- reflector, row i of R, norms and the next pivot: the same in
     // every CTA
