@@ -570,7 +570,7 @@ def main():
                         "unit": "TFLOP/s", "frac": a / peak64 if a else None,
                         "flops_per_step": flops, "ms_per_step": ms, "launches": launches}
             rooflines["id"] = fp64_line(
-                "id_onchip_kernel / id_kernel (entry generation, pivoted QR, T)",
+                "id_tile_kernel / id_cluster_kernel / id_kernel (entry generation, pivoted QR, T)",
                 st["id_flops"], st["id_ms"], st["id_launches"])
             rooflines["id"]["algorithmic_hbm_bytes"] = st["id_bytes"]
             rooflines["id"]["traffic_per_launch"] = traffic_from_profile(args.workload)

@@ -1731,7 +1731,7 @@ cudaError_t launch_border_rhs(const double* Pred, int nr, int nb, const double* 
 // w - (X^{-1} U) alpha, with X^{-1} w in x already and X^{-1} U kept by the
 // factorization, so that the diagonal blocks are read once a solve (of eight
 // holes and 65,536 dofs: this kernel and the two above 19 us, the products,
-// copies, gathers and second diagonal solve they replace about 105 us).
+// gathers and second diagonal solve they replace 73 us).
 __global__ void __launch_bounds__(kBorderThreads)
     border_apply_kernel(const double* __restrict__ dinv, int nr, int nb,
                         const int* __restrict__ allred, const int* __restrict__ allskel, int ns,

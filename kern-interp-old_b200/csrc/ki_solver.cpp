@@ -900,8 +900,10 @@ int Solver::id_launch(int level, PendingLevel* pl) {
   if (order.empty()) return 0;
   // A box in registers takes more CTAs than one in shared memory (160 KB of
   // an SM's registers hold matrix entries, 220 KB of its shared memory) but
-  // is done sooner, so a level that fits the GPU in registers takes them and
-  // a fuller one the smaller clusters.
+  // is done sooner, so a level that fits the GPU in registers takes them (9
+  // boxes of 976 x 58: 0.12 ms, in shared memory 0.17) and a fuller one the
+  // smaller clusters (705 Stokes boxes of 924 x 122 and less: 3.2 ms, in
+  // registers 5.6).
   int ctas = 0;
   for (int q : order) ctas += all[q].g % 100;
   if (ctas > num_sms_)

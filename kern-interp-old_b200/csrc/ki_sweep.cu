@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kSweepThreads) sweep_kernel(SweepParams P, int
 // cluster per box (see wide_rows).  Every CTA gathers the whole vector,
 // forms its rows of the first product, hands them to the others and forms
 // its rows of the second.  A 65,536-dof Stokes problem's four boxes of level
-// 1: 40 us -> 12 us a sweep, the sixteen of level 2: 22 us -> 11 us (one CTA
+// 1: 28 us -> 15 us a sweep, the sixteen of level 2: 16 us -> 11 us (one CTA
 // per box before).
 template <int MODE>
 __global__ void __launch_bounds__(kWideThreads) sweep_wide_kernel(SweepParams P) {
@@ -527,7 +527,7 @@ cudaError_t launch_transposed_up(const SweepParams& p, cudaStream_t s) {
 namespace {
 // The diagonal step of a few large boxes, one right-hand side: a cluster per
 // box, x_r <- X^{-1} x_r by rows (ys = 0 - X^{-1} xs, stored negated): one
-// box of that problem 34 us -> 11 us.
+// box of that problem 24 us -> 11 us.
 template <bool TRANS>
 __global__ void __launch_bounds__(kWideThreads) diag_wide_kernel(SweepParams P) {
   wait_prior_grid();
