@@ -250,7 +250,6 @@ namespace {
 // small factorization's level loop).
 struct AuxSet {
   int dev = -1;
-  bool high = false;  // the decoupling's streams have the highest priority
   cudaStream_t d = nullptr;
   cudaEvent_t ev_id[2] = {}, ev_dec = nullptr, fork = nullptr;
   cudaStream_t id[3] = {};
@@ -301,7 +300,6 @@ Solver::~Solver() {
     static_assert(kIdStreams == 3 && kDecStreams == 3, "AuxSet holds three of each");
     AuxSet a;
     cudaGetDevice(&a.dev);
-    a.high = opt_.sketch_id;
     a.d = dstream_;
     a.ev_id[0] = ev_id_[0];
     a.ev_id[1] = ev_id_[1];
@@ -488,7 +486,7 @@ int Solver::begin_factor(cudaEvent_t* ev0) {
       std::lock_guard<std::mutex> lk(g_aux_mu);
       auto& fl = aux_free();
       for (size_t i = 0; i < fl.size(); i++)
-        if (fl[i].dev == dev && fl[i].high == opt_.sketch_id) {
+        if (fl[i].dev == dev) {
           const AuxSet a = fl[i];
           fl.erase(fl.begin() + static_cast<long>(i));
           dstream_ = a.d;
@@ -514,13 +512,7 @@ int Solver::begin_factor(cudaEvent_t* ev0) {
         }
     }
     if (!dstream_) {
-      // A preconditioner's factorization waits for its chain of
-      // decouplings (its sketched IDs finish early), a reference one for its
-      // IDs: the decouplings' blocks go first only in the former.
-      int lowest = 0, highest = 0;
-      KI_CUDA(cudaDeviceGetStreamPriorityRange(&lowest, &highest));
-      const int prio = opt_.sketch_id ? highest : lowest;
-      KI_CUDA(cudaStreamCreateWithPriority(&dstream_, cudaStreamNonBlocking, prio));
+      KI_CUDA(cudaStreamCreateWithFlags(&dstream_, cudaStreamNonBlocking));
       KI_CUDA(cudaEventCreateWithFlags(&ev_id_[0], cudaEventDisableTiming));
       KI_CUDA(cudaEventCreateWithFlags(&ev_id_[1], cudaEventDisableTiming));
       KI_CUDA(cudaEventCreateWithFlags(&ev_dec_, cudaEventDisableTiming));
@@ -531,7 +523,7 @@ int Solver::begin_factor(cudaEvent_t* ev0) {
       }
       KI_CUDA(cudaEventCreateWithFlags(&dl_fork_, cudaEventDisableTiming));
       for (int i = 0; i < kDecStreams; i++) {
-        KI_CUDA(cudaStreamCreateWithPriority(&dl_streams_[i], cudaStreamNonBlocking, prio));
+        KI_CUDA(cudaStreamCreateWithFlags(&dl_streams_[i], cudaStreamNonBlocking));
         KI_CUDA(cudaEventCreateWithFlags(&dl_join_[i], cudaEventDisableTiming));
       }
       KI_CUDA(cudaStreamCreateWithFlags(&bstream_, cudaStreamNonBlocking));
@@ -736,18 +728,15 @@ int Solver::finish_factor(cudaEvent_t ev0) {
     for (int level = L - 1; level > 0 && !rc; level--) {
       auto next = std::make_unique<PendingLevel>();
       const bool more = level > 1 && !(level == 2 && level1_stays());
-      // the deepest level's decouplings, when they fill the GPU more than
-      // once, are the head of the chain a preconditioner's factorization
-      // waits for: queued before the next IDs are prepared (every later
-      // level's wait for the ones below in any case)
-      const bool dec_first = opt_.sketch_id && level == L - 1 &&
-                             static_cast<int>(cur->comp.size()) > 2 * num_sms_;
-      if (dec_first) rc = decouple_level(cur.get());
-      if (!rc && more) {
+      // (the IDs first at every level: with the decoupling in registers they
+      // are the longer chain in either mode.  The deepest level's decoupling
+      // first, as suited a slower one: 5.31 ms against 5.12 ms for 65,536
+      // Stokes dofs in preconditioner mode)
+      if (more) {
         rc = id_launch(level - 1, next.get());
         refreshed = level - 1;
       }
-      if (!rc && !dec_first) rc = decouple_level(cur.get());
+      if (!rc) rc = decouple_level(cur.get());
       if (!rc && more) rc = id_finish(next.get());
       if (!more) break;
       cur = std::move(next);
