@@ -46,8 +46,8 @@ __device__ __forceinline__ double upd_lookup(const int* bid, const int* bpos,
 __host__ __device__ inline int frag_ld(int n) { return n + ((4 - n % 8) + 8) % 8; }
 
 // The CTA's product op(A) op(B) (m x n, inner kk) on the FP64 tensor cores,
-// both operands in shared memory with a frag_ld stride; out(i, j, v)
-// receives every entry.  A warp computes 16 x 16 blocks (2 x 2 DMMA blocks)
+// the operands in shared memory with a frag_ld stride (X_rr of L's
+// correction: in global memory); out(i, j, v) receives every entry.  A warp computes 16 x 16 blocks (2 x 2 DMMA blocks)
 // straight from the operands: no staging, no barriers.
 template <bool TA, bool TB, class Out>
 __device__ __forceinline__ void cta_mma(const double* A, int lda, const double* B, int ldb, int m,
@@ -207,22 +207,19 @@ __device__ __forceinline__ int cta_gj_regs(double* X, int ld, int r, double* col
 }
 
 // Shared memory of a box: K_BN (in place K_r_sn, K_sn_r, X_rr and its
-// inverse), T and later L, the pivot column twice, pivots, per-dof ints; with
-// L's correction the staging tile of a product with an operand in global
-// memory.
+// inverse), T and later L, the pivot column twice, pivots, per-dof ints.
 struct DecLayout {
   int ldn, ldk;
-  size_t tl, tile, colj, ints, bytes;  // offsets in doubles, total bytes
+  size_t tl, colj, ints, bytes;  // offsets in doubles, total bytes
 };
-__host__ __device__ inline DecLayout dec_layout(int n, int k, bool correct) {
+__host__ __device__ inline DecLayout dec_layout(int n, int k) {
   DecLayout d;
   const int r = n - k;
   d.ldn = frag_ld(n);
   d.ldk = frag_ld(k);
   d.tl = static_cast<size_t>(n) * d.ldn;
   const size_t t = static_cast<size_t>(d.ldk) * r, nodes = 8 * static_cast<size_t>(n);
-  d.tile = d.tl + (((t > nodes ? t : nodes) + 1) & ~static_cast<size_t>(1));
-  d.colj = d.tile + (correct ? kGemmTileDoubles : 0);
+  d.colj = d.tl + (((t > nodes ? t : nodes) + 1) & ~static_cast<size_t>(1));
   d.ints = d.colj + 2 * 160;
   d.bytes = sizeof(double) * d.ints + sizeof(int) * (5 * static_cast<size_t>(n) + 4);
   return d;
@@ -235,7 +232,7 @@ __global__ void __launch_bounds__(kDecThreads, MINB) decouple_kernel(DecParams P
   extern __shared__ __align__(16) double dsm[];
   const DecTask tk = P.tasks[blockIdx.x];
   const int n = tk.n, k = tk.k, r = n - k;
-  const DecLayout lay = dec_layout(n, k, !FAST);
+  const DecLayout lay = dec_layout(n, k);
   const int ldn = lay.ldn, ldk = lay.ldk;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double* K = dsm;
@@ -311,16 +308,18 @@ __global__ void __launch_bounds__(kDecThreads, MINB) decouple_kernel(DecParams P
   cta_mma<false, false>(Krs, ldn, TL, ldk, r, r, k, minus(Krr));
   cta_mma<false, false>(Kss, ldn, TL, ldk, k, r, k, minus(Ksr));
   __syncthreads();
-  if (!FAST)  // X_rr itself, for L's correction
+  auto store_x = [&]() {
     for (int c = warp; c < r; c += kDecThreads / 32)
       for (int i = lane; i < r; i += 32)
-        tk.X0[i + static_cast<size_t>(r) * c] = Krr[i + static_cast<size_t>(ldn) * c];
+        tk.X[i + static_cast<size_t>(r) * c] = Krr[i + static_cast<size_t>(ldn) * c];
+  };
+  // (L's correction needs X_rr itself: until then it waits in the place of
+  // its inverse)
+  if (!FAST) store_x();
   const int info = cta_gj_regs<CW, RS>(Krr, ldn, r, colj, sp, prow, pinv);
   if (info && threadIdx.x == 0) atomicExch(P.status, 1);
   for (int j = threadIdx.x; j < r; j += kDecThreads) tk.piv[j] = prow[j];
-  for (int c = warp; c < r; c += kDecThreads / 32)
-    for (int i = lane; i < r; i += 32)
-      tk.X[i + static_cast<size_t>(r) * c] = Krr[i + static_cast<size_t>(ldn) * c];
+  if (FAST) store_x();
   // U = X^{-1} K_r_sn,  L = K_sn_r X^{-1}  (in T's place)
   cta_mma<false, false>(Krr, ldn, Krs, ldn, r, k, r, [&](int i, int j, double v) {
     tk.U[i + static_cast<size_t>(r) * j] = v;
@@ -330,7 +329,9 @@ __global__ void __launch_bounds__(kDecThreads, MINB) decouple_kernel(DecParams P
   });
   __syncthreads();
   if (!FAST) {
-    cta_gemm_tiled(Ksr, ldn, Ksr, ldn, TL, ldk, false, tk.X0, r, false, k, r, r, dsm + lay.tile);
+    cta_mma<false, false>(TL, ldk, tk.X, r, k, r, r, minus(Ksr));
+    __syncthreads();
+    store_x();
     cta_mma<false, false>(Ksr, ldn, Krr, ldn, k, r, r, [&](int i, int j, double v) {
       TL[i + static_cast<size_t>(ldk) * j] += v;
     });
@@ -384,7 +385,13 @@ __global__ void acc_finish_kernel(double* acc, int k, const int* perm, const int
 
 }  // namespace
 
-cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* status,
+// K_BN (n x n), the LU's flags, and X_rr in reference mode
+size_t decouple_large_scratch(int n, int k, bool fast) {
+  const size_t r = static_cast<size_t>(n) - k;
+  return static_cast<size_t>(n) * n + kLuSyncInts + (fast ? 0 : r * r);
+}
+
+cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* status, bool fast,
                            cudaStream_t s) {
   const int n = tk.n, k = tk.k, r = n - k;
   const long long nn = static_cast<long long>(n) * n;
@@ -413,8 +420,8 @@ cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* s
     return e;
   if ((e = cudaMemcpyAsync(Ksnr, tk.L, sizeof(double) * r * k, cudaMemcpyDeviceToDevice, s)))
     return e;
-  if (tk.X0 && (e = cudaMemcpyAsync(tk.X0, tk.X, sizeof(double) * r * r,
-                                    cudaMemcpyDeviceToDevice, s)))
+  double* X0 = tk.K + nn + kLuSyncInts;  // X_rr, for L's correction
+  if (!fast && (e = cudaMemcpyAsync(X0, tk.X, sizeof(double) * r * r, cudaMemcpyDeviceToDevice, s)))
     return e;
   if ((e = dense_lu(tk.X, r, r, tk.piv, status, s, reinterpret_cast<int*>(tk.K + nn)))) return e;
   count_launches(1);
@@ -429,8 +436,8 @@ cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* s
   if ((e = launch_gemm_tiled(tk.L, k, nullptr, 0, Ksnr, k, false, tk.X, r, false, k, r, r, 1.0,
                              s)))
     return e;
-  if (tk.X0) {
-    if ((e = launch_gemm_sub(Ksnr, k, Ksnr, k, tk.L, k, false, tk.X0, r, false, k, r, r, s)))
+  if (!fast) {
+    if ((e = launch_gemm_sub(Ksnr, k, Ksnr, k, tk.L, k, false, X0, r, false, k, r, r, s)))
       return e;
     if ((e = launch_gemm_tiled(tk.L, k, tk.L, k, Ksnr, k, false, tk.X, r, false, k, r, r, 1.0, s)))
       return e;
@@ -462,7 +469,7 @@ cudaError_t launch_class(const DecParams& p, bool fast, size_t smem, cudaStream_
 }
 }  // namespace
 
-size_t decouple_smem_bytes(int n, int k, bool fast) { return dec_layout(n, k, !fast).bytes; }
+size_t decouple_smem_bytes(int n, int k) { return dec_layout(n, k).bytes; }
 
 int decouple_class(int n, int k) {
   const int r = n - k;

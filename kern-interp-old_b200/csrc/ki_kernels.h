@@ -141,13 +141,12 @@ struct DecTask {
   const int* bpos;       // per active position: row inside that block
   const UpdBlock* blocks;
   const double* T;       // k x r, ld k (from the ID)
-  double* K;             // scratch n x n + kLuSyncInts (boxes too large for shared memory)
+  double* K;             // scratch of decouple_large_scratch doubles (large boxes only)
   double* L;             // k x r, ld k
   double* U;             // r x k, ld r
   double* X;             // X_rr^{-1}, r x r, ld r (written by the decoupling)
   double* acc;           // accumulated update on the skeleton, k x k
   int* piv;              // r ints of scratch (pivots of the inversion)
-  double* X0;            // r x r scratch that keeps X_rr for L's correction (null: none)
 };
 
 struct DecParams {
@@ -164,11 +163,13 @@ struct DecParams {
 // preconditioner's).  Boxes of class -1 or past 227 KB go through
 // decouple_large instead.
 int decouple_class(int n, int k);
-size_t decouple_smem_bytes(int n, int k, bool fast);
+size_t decouple_smem_bytes(int n, int k);
 cudaError_t launch_decouple(const DecParams& p, int cls, bool fast, size_t smem, cudaStream_t s);
 // The same decoupling for one large box as a sequence of GPU-wide kernels
-// (tk is the host copy of the box's descriptor; tk.K must hold n x n).
-cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* status,
+// (tk is the host copy of the box's descriptor; tk.K holds
+// decouple_large_scratch doubles).
+size_t decouple_large_scratch(int n, int k, bool fast);
+cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* status, bool fast,
                            cudaStream_t s);
 
 // Dense assembly of the top-level skeleton matrix K(allskel, allskel) minus

@@ -1281,11 +1281,11 @@ int Solver::decouple_boxes(PendingLevel* pl) {
   });
   const bool fast = opt_.sketch_id;
   auto large_box = [&](int n, int k) {
-    return decouple_class(n, k) < 0 || decouple_smem_bytes(n, k, fast) > 227 * 1024;
+    return decouple_class(n, k) < 0 || decouple_smem_bytes(n, k) > 227 * 1024;
   };
   std::vector<long long> bid_off(ncomp + 1, 0), tab_off(ncomp + 1, 0);
   long long scratch_total = 0;
-  std::vector<long long> k_off(ncomp), x0_off(ncomp);
+  std::vector<long long> k_off(ncomp);
   std::vector<size_t> f_off(ncomp), p_off(ncomp);
   int n_max = 0;
   size_t fac_total = 0, piv_total = 0;
@@ -1297,13 +1297,10 @@ int Solver::decouple_boxes(PendingLevel* pl) {
     tab_off[t + 1] = tab_off[t] + static_cast<long long>(blk[t].size());
     k_off[t] = scratch_total;
     if (large_box(n, k)) {
-      // n x n, then the LU's flags (kLuSyncInts ints)
-      scratch_total += static_cast<long long>(n) * n + kLuSyncInts;
+      scratch_total += static_cast<long long>(decouple_large_scratch(n, k, fast));
     } else {
       n_max = std::max(n_max, n);
     }
-    x0_off[t] = scratch_total;
-    if (!opt_.sketch_id) scratch_total += static_cast<long long>(r) * r;
     f_off[t] = fac_total;
     p_off[t] = piv_total;
     fac_total += static_cast<size_t>(k) * r * 2 + static_cast<size_t>(r) * r +
@@ -1337,7 +1334,7 @@ int Solver::decouple_boxes(PendingLevel* pl) {
       large.push_back(t);
       continue;
     }
-    const size_t bytes = decouple_smem_bytes(n, k, fast) + 1024;
+    const size_t bytes = decouple_smem_bytes(n, k) + 1024;
     key[t] = 4 * decouple_class(n, k) +
              3 - static_cast<int>(std::min<size_t>(3, static_cast<size_t>(smem_per_sm_) / bytes));
     small.push_back(t);
@@ -1391,7 +1388,6 @@ int Solver::decouple_boxes(PendingLevel* pl) {
       d.X = bd.X;
       d.acc = bd.acc;
       d.piv = bd.piv;
-      d.X0 = opt_.sketch_id ? nullptr : scr + x0_off[t];
       if (i < nsmall) reinterpret_cast<DecTask*>(st)[i] = d;
     }
   });
@@ -1429,7 +1425,7 @@ int Solver::decouple_boxes(PendingLevel* pl) {
     size_t smem = 0;
     const int ka = key[small[a]];
     while (b < nsmall && key[small[b]] == ka) {
-      smem = std::max(smem, decouple_smem_bytes(dt[b].n, dt[b].k, fast));
+      smem = std::max(smem, decouple_smem_bytes(dt[b].n, dt[b].k));
       b++;
     }
     DecParams dpc = dp;
@@ -1444,7 +1440,7 @@ int Solver::decouple_boxes(PendingLevel* pl) {
   for (int t = nsmall; t < ncomp; t++) {
     cudaStream_t cs;
     if (side_stream(&cs)) return -2;
-    KI_CUDA(decouple_large(dt[t], opt_.pde, d_nodes_, d_status_, cs));
+    KI_CUDA(decouple_large(dt[t], opt_.pde, d_nodes_, d_status_, fast, cs));
     n_large = std::max(n_large, dt[t].n);
   }
   for (int i = 0; i < kDecStreams; i++)
