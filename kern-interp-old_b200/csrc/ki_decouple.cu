@@ -30,6 +30,7 @@ namespace kib {
 namespace {
 
 constexpr int kDecThreads = 256;
+constexpr size_t kDecSmemMax = 227 * 1024;
 
 __device__ __forceinline__ double upd_lookup(const int* bid, const int* bpos,
                                              const UpdBlock* blocks, int a, int b) {
@@ -207,18 +208,19 @@ __device__ __forceinline__ int cta_gj_regs(double* X, int ld, int r, double* col
 }
 
 // Shared memory of a box: K_BN (in place K_r_sn, K_sn_r, X_rr and its
-// inverse), T and later L, the pivot column twice, pivots, per-dof ints.
+// inverse), T and later L (tl: unless they stay in global memory), the pivot
+// column twice, pivots, per-dof ints.
 struct DecLayout {
   int ldn, ldk;
   size_t tl, colj, ints, bytes;  // offsets in doubles, total bytes
 };
-__host__ __device__ inline DecLayout dec_layout(int n, int k) {
+__host__ __device__ inline DecLayout dec_layout(int n, int k, bool tl) {
   DecLayout d;
   const int r = n - k;
   d.ldn = frag_ld(n);
-  d.ldk = frag_ld(k);
+  d.ldk = tl ? frag_ld(k) : k;
   d.tl = static_cast<size_t>(n) * d.ldn;
-  const size_t t = static_cast<size_t>(d.ldk) * r, nodes = 8 * static_cast<size_t>(n);
+  const size_t t = tl ? static_cast<size_t>(d.ldk) * r : 0, nodes = 8 * static_cast<size_t>(n);
   d.colj = d.tl + (((t > nodes ? t : nodes) + 1) & ~static_cast<size_t>(1));
   d.ints = d.colj + 2 * 160;
   d.bytes = sizeof(double) * d.ints + sizeof(int) * (5 * static_cast<size_t>(n) + 4);
@@ -226,17 +228,24 @@ __host__ __device__ inline DecLayout dec_layout(int n, int k) {
 }
 
 // FAST: entries by contracted arithmetic (a preconditioner's, whose sketched
-// IDs use it too); else the reference's bits, and L corrected.
-template <int CW, int RS, int MINB, bool FAST>
+// IDs use it too); else the reference's bits, and L corrected.  TL: T is
+// copied to shared memory, where L takes its place; else, for boxes whose
+// K_BN leaves no room for it (149 dofs and more, by rank), the products read
+// T, and L as it is made, in global memory (from L1: a warp's fragment is
+// eight runs of four entries).  Sent through decouple_large instead, as the
+// only alternative, such boxes cost 17 launches each: 16,384-node star, 160
+// dofs a leaf, 4.65 ms against 2.96 ms, 200 a leaf 7.26 against 5.44 ms.
+template <int CW, int RS, int MINB, bool FAST, bool TL>
 __global__ void __launch_bounds__(kDecThreads, MINB) decouple_kernel(DecParams P) {
   extern __shared__ __align__(16) double dsm[];
   const DecTask tk = P.tasks[blockIdx.x];
   const int n = tk.n, k = tk.k, r = n - k;
-  const DecLayout lay = dec_layout(n, k);
+  const DecLayout lay = dec_layout(n, k, TL);
   const int ldn = lay.ldn, ldk = lay.ldk;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double* K = dsm;
-  double* TL = dsm + lay.tl;
+  const double* T = TL ? dsm + lay.tl : tk.T;
+  double* L = TL ? dsm + lay.tl : tk.L;
   double* colj = dsm + lay.colj;
   int* prow = reinterpret_cast<int*>(dsm + lay.ints);  // n
   int* pinv = prow + n;                                 // n
@@ -248,7 +257,7 @@ __global__ void __launch_bounds__(kDecThreads, MINB) decouple_kernel(DecParams P
   // ---- K_BN in pivot order: a lane keeps its row's node record and block,
   // the columns' records pass by broadcast, four at a time (their update
   // entries are loads from global memory)
-  Node* nd = reinterpret_cast<Node*>(TL);
+  Node* nd = reinterpret_cast<Node*>(dsm + lay.tl);
   const int sh = P.pde == kStokes ? 1 : 0;
   for (int a = threadIdx.x; a < n; a += kDecThreads) {
     const int pa = tk.perm[a], d = tk.act[pa];
@@ -288,10 +297,12 @@ __global__ void __launch_bounds__(kDecThreads, MINB) decouple_kernel(DecParams P
     }
   }
   __syncthreads();
-  for (int c = warp; c < r; c += kDecThreads / 32)
-    for (int l = lane; l < k; l += 32)
-      TL[l + static_cast<size_t>(ldk) * c] = tk.T[l + static_cast<size_t>(k) * c];
-  __syncthreads();
+  if (TL) {
+    for (int c = warp; c < r; c += kDecThreads / 32)
+      for (int l = lane; l < k; l += 32)
+        L[l + static_cast<size_t>(ldk) * c] = tk.T[l + static_cast<size_t>(k) * c];
+    __syncthreads();
+  }
   double* Kss = K;
   double* Krs = K + k;
   double* Ksr = K + static_cast<size_t>(ldn) * k;
@@ -302,11 +313,11 @@ __global__ void __launch_bounds__(kDecThreads, MINB) decouple_kernel(DecParams P
   // K_r_sn = K_rs - T^T K_ss,  X = (K_rr - T^T K_sr) - K_r_sn T,  K_sn_r =
   // K_sr - K_ss T, each in place (an entry is read as C only by the thread
   // that replaces it)
-  cta_mma<true, false>(TL, ldk, Kss, ldn, r, k, k, minus(Krs));
-  cta_mma<true, false>(TL, ldk, Ksr, ldn, r, r, k, minus(Krr));
+  cta_mma<true, false>(T, ldk, Kss, ldn, r, k, k, minus(Krs));
+  cta_mma<true, false>(T, ldk, Ksr, ldn, r, r, k, minus(Krr));
   __syncthreads();
-  cta_mma<false, false>(Krs, ldn, TL, ldk, r, r, k, minus(Krr));
-  cta_mma<false, false>(Kss, ldn, TL, ldk, k, r, k, minus(Ksr));
+  cta_mma<false, false>(Krs, ldn, T, ldk, r, r, k, minus(Krr));
+  cta_mma<false, false>(Kss, ldn, T, ldk, k, r, k, minus(Ksr));
   __syncthreads();
   auto store_x = [&]() {
     for (int c = warp; c < r; c += kDecThreads / 32)
@@ -320,28 +331,29 @@ __global__ void __launch_bounds__(kDecThreads, MINB) decouple_kernel(DecParams P
   if (info && threadIdx.x == 0) atomicExch(P.status, 1);
   for (int j = threadIdx.x; j < r; j += kDecThreads) tk.piv[j] = prow[j];
   if (FAST) store_x();
-  // U = X^{-1} K_r_sn,  L = K_sn_r X^{-1}  (in T's place)
+  // U = X^{-1} K_r_sn,  L = K_sn_r X^{-1}  (TL: in T's place)
   cta_mma<false, false>(Krr, ldn, Krs, ldn, r, k, r, [&](int i, int j, double v) {
     tk.U[i + static_cast<size_t>(r) * j] = v;
   });
   cta_mma<false, false>(Ksr, ldn, Krr, ldn, k, r, r, [&](int i, int j, double v) {
-    TL[i + static_cast<size_t>(ldk) * j] = v;
+    L[i + static_cast<size_t>(ldk) * j] = v;
   });
   __syncthreads();
   if (!FAST) {
-    cta_mma<false, false>(TL, ldk, tk.X, r, k, r, r, minus(Ksr));
+    cta_mma<false, false>(L, ldk, tk.X, r, k, r, r, minus(Ksr));
     __syncthreads();
     store_x();
     cta_mma<false, false>(Ksr, ldn, Krr, ldn, k, r, r, [&](int i, int j, double v) {
-      TL[i + static_cast<size_t>(ldk) * j] += v;
+      L[i + static_cast<size_t>(ldk) * j] += v;
     });
     __syncthreads();
   }
-  for (int c = warp; c < r; c += kDecThreads / 32)
-    for (int l = lane; l < k; l += 32)
-      tk.L[l + static_cast<size_t>(k) * c] = TL[l + static_cast<size_t>(ldk) * c];
+  if (TL)
+    for (int c = warp; c < r; c += kDecThreads / 32)
+      for (int l = lane; l < k; l += 32)
+        tk.L[l + static_cast<size_t>(k) * c] = L[l + static_cast<size_t>(ldk) * c];
   // acc = update(s, s) + L K_r_sn
-  cta_mma<false, false>(TL, ldk, Krs, ldn, k, k, r, [&](int i, int j, double v) {
+  cta_mma<false, false>(L, ldk, Krs, ldn, k, k, r, [&](int i, int j, double v) {
     const int bi = sbid[i];
     double up = 0.0;
     if (bi >= 0 && bi == sbid[j])
@@ -451,39 +463,45 @@ cudaError_t decouple_large(const DecTask& tk, int pde, const Node* nodes, int* s
 
 namespace {
 // The register tile of X_rr's inversion by r, and the CTAs of it an SM's
-// registers hold.
-template <int CW, int RS, int MINB>
-cudaError_t launch_class(const DecParams& p, bool fast, size_t smem, cudaStream_t s) {
-  const void* fn = fast ? reinterpret_cast<const void*>(&decouple_kernel<CW, RS, MINB, true>)
-                        : reinterpret_cast<const void*>(&decouple_kernel<CW, RS, MINB, false>);
-  cudaError_t e = raise_func_attr(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem));
+// registers hold (without TL: its shared memory holds one).
+template <int CW, int RS, int MINB, bool FAST, bool TL>
+cudaError_t launch_class(const DecParams& p, size_t smem, cudaStream_t s) {
+  const cudaError_t e = raise_func_attr(
+      reinterpret_cast<const void*>(&decouple_kernel<CW, RS, MINB, FAST, TL>),
+      cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   count_launches(1);
-  if (fast) {
-    decouple_kernel<CW, RS, MINB, true><<<p.ntasks, kDecThreads, smem, s>>>(p);
-  } else {
-    decouple_kernel<CW, RS, MINB, false><<<p.ntasks, kDecThreads, smem, s>>>(p);
-  }
+  decouple_kernel<CW, RS, MINB, FAST, TL><<<p.ntasks, kDecThreads, smem, s>>>(p);
   return cudaGetLastError();
+}
+template <bool FAST>
+cudaError_t launch_any(const DecParams& p, int cls, size_t smem, cudaStream_t s) {
+  switch (cls) {
+    case 0: return launch_class<8, 2, 3, FAST, true>(p, smem, s);
+    case 1: return launch_class<12, 3, 2, FAST, true>(p, smem, s);
+    case 2: return launch_class<20, 5, 1, FAST, true>(p, smem, s);
+    case 3: return launch_class<8, 2, 1, FAST, false>(p, smem, s);
+    case 4: return launch_class<12, 3, 1, FAST, false>(p, smem, s);
+    case 5: return launch_class<20, 5, 1, FAST, false>(p, smem, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 }  // namespace
 
-size_t decouple_smem_bytes(int n, int k) { return dec_layout(n, k).bytes; }
-
 int decouple_class(int n, int k) {
-  const int r = n - k;
-  return r <= 64 ? 0 : r <= 96 ? 1 : r <= 160 ? 2 : -1;
+  const int r = n - k, tile = r <= 64 ? 0 : r <= 96 ? 1 : r <= 160 ? 2 : -1;
+  if (tile < 0) return -1;
+  if (dec_layout(n, k, true).bytes <= kDecSmemMax) return tile;
+  return dec_layout(n, k, false).bytes <= kDecSmemMax ? 3 + tile : -1;
+}
+
+size_t decouple_smem_bytes(int n, int k) {
+  return dec_layout(n, k, decouple_class(n, k) < 3).bytes;
 }
 
 cudaError_t launch_decouple(const DecParams& p, int cls, bool fast, size_t smem, cudaStream_t s) {
   if (p.ntasks == 0) return cudaSuccess;
-  switch (cls) {
-    case 0: return launch_class<8, 2, 3>(p, fast, smem, s);
-    case 1: return launch_class<12, 3, 2>(p, fast, smem, s);
-    case 2: return launch_class<20, 5, 1>(p, fast, smem, s);
-    default: return cudaErrorInvalidValue;
-  }
+  return fast ? launch_any<true>(p, cls, smem, s) : launch_any<false>(p, cls, smem, s);
 }
 
 cudaError_t launch_assemble_top(int pde, const Node* nodes, const int* dofs, int n,

@@ -157,11 +157,12 @@ struct DecParams {
   int* status;  // set nonzero on an exactly zero pivot
 };
 
-// One launch for boxes of one class (decouple_class: the size of X_rr's
-// register tile; -1: too large for a CTA) with `smem` bytes, the largest
-// decouple_smem_bytes of them.  fast: contracted entries, L not corrected (a
-// preconditioner's).  Boxes of class -1 or past 227 KB go through
-// decouple_large instead.
+// One launch for boxes of one class with `smem` bytes, the largest
+// decouple_smem_bytes of them.  decouple_class: the size of X_rr's register
+// tile (r <= 64, 96, 160: 0, 1, 2), + 3 where T and L stay in global memory;
+// -1: too large for a CTA (more than 164 dofs, or more than 160 of them
+// redundant), through decouple_large.  fast: contracted entries, L not
+// corrected (a preconditioner's).
 int decouple_class(int n, int k);
 size_t decouple_smem_bytes(int n, int k);
 cudaError_t launch_decouple(const DecParams& p, int cls, bool fast, size_t smem, cudaStream_t s);

@@ -1280,9 +1280,7 @@ int Solver::decouple_boxes(PendingLevel* pl) {
     }
   });
   const bool fast = opt_.sketch_id;
-  auto large_box = [&](int n, int k) {
-    return decouple_class(n, k) < 0 || decouple_smem_bytes(n, k) > 227 * 1024;
-  };
+  auto large_box = [&](int n, int k) { return decouple_class(n, k) < 0; };
   std::vector<long long> bid_off(ncomp + 1, 0), tab_off(ncomp + 1, 0);
   long long scratch_total = 0;
   std::vector<long long> k_off(ncomp);
