@@ -892,12 +892,17 @@ int Solver::id_launch(int level, PendingLevel* pl) {
   // is done sooner, so a level that fits the GPU in registers takes them (9
   // boxes of 976 x 58: 0.12 ms, in shared memory 0.17) and a fuller one the
   // smaller clusters (705 Stokes boxes of 924 x 122 and less: 3.2 ms, in
-  // registers 5.6).
-  int ctas = 0;
-  for (int q : order) ctas += all[q].g % 100;
-  if (ctas > num_sms_)
-    for (Cand& c : all)
-      if (c.g_slab && c.g >= kTile && c.g_slab % 100 < c.g % 100) c.g = c.g_slab;
+  // registers 5.6).  A tree's own boxes decide, not the whole level of a
+  // forest: the two add a column's rows in different orders, and a problem
+  // keeps in a batch the pivots it has alone.
+  std::vector<int> ctas(std::max<size_t>(1, tree.roots.size()), 0);
+  for (int q : order) ctas[tree.boxes[ids[q]].tree] += all[q].g % 100;
+  for (int q : order) {
+    Cand& c = all[q];
+    if (ctas[tree.boxes[ids[q]].tree] > num_sms_ && c.g_slab && c.g >= kTile &&
+        c.g_slab % 100 < c.g % 100)
+      c.g = c.g_slab;
+  }
   // grouped by cluster size, the group holding the widest ID matrix first
   // (its launch then takes SMs before the many-box launch fills them: the
   // few big boxes are each level's longest tasks), and inside a group the
