@@ -96,15 +96,23 @@ def peaks():
 
 def traffic_from_profile(workload):
     """DRAM bytes per ID launch (read + write, averaged over the ID launches of
-    one factorization) from the committed ncu summary of this workload."""
+    one factorization) from the committed ncu summary of this workload; None
+    if that measured a kernel that the sources no longer have."""
+    import glob
     import re
     path = os.path.join(ROOT, "profiles", "id_kernel_%s.txt" % workload)
     try:
         with open(path) as f:
-            m = re.search(r"^dram_bytes_per_id_launch:\s*([0-9.eE+]+)", f.read(), re.M)
-        return float(m.group(1)) if m else None
+            text = f.read()
     except OSError:
         return None
+    m = re.search(r"^dram_bytes_per_id_launch:\s*([0-9.eE+]+)", text, re.M)
+    src = "".join(open(p).read() for p in
+                  glob.glob(os.path.join(ROOT, "kern-interp-old_b200", "csrc", "*.cu")))
+    kernels = set(re.findall(r"^ +(id_\w+)<", text, re.M))
+    if not m or not kernels or any(not re.search(r"\b%s\(" % k, src) for k in kernels):
+        return None
+    return float(m.group(1))
 
 
 def fp64_peak_tflops(dev):
