@@ -1220,7 +1220,7 @@ __global__ void __launch_bounds__(kOcThreads, 1) id_cluster_kernel(IdParams P) {
   candidates(n);  // (each thread reads back its own norms)
   __syncthreads();
   int pick = chosen(kOcWarps);
-  e0 = static_cast<int>(__double_as_longlong(vn1[pick & 0xffff]) >> 52);
+  e0 = static_cast<int>(cand_key(vn1[pick & 0xffff]) >> 52);
 
   const double tol3z = sqrt(0.5 * 2.220446049250313e-16);
   // lanes per column and columns per group: a warp carries four columns
