@@ -6,7 +6,7 @@
 //
 // The reference forms K_domain as a dense |targets| x N matrix (16 GB for a
 // 350^2 grid on 16,384 nodes) and multiplies it.  Here each thread owns one
-// target and sweeps the source nodes staged in shared memory, forming the
+// or two targets and sweeps the source nodes staged in shared memory, forming the
 // entries on the fly (FP64, reciprocal by a refined hardware estimate, so the
 // sums agree with the exact entries to FP64 rounding); the sources are split
 // across CTAs when there are too few targets to fill the GPU, and a finish
@@ -36,65 +36,68 @@ constexpr double kDomainEps = 1e-2;  // cubic_boundary.cpp:185, circle.cpp:37
 //   Laplace:          a = -(w / 2 pi) mu (n_x, n_y)
 //   Laplace-Neumann:  a0 = (w / 2 pi) mu        (forward entry (w/2pi) log|r|)
 //   Stokes:           a = (w / pi) (n_x, n_y), density (mu_0, mu_1)
-// A thread owns two targets of a block's 256, 128 apart, as in the operator
-// product: bound by the FP64 pipe.  live, if given, is the number of points
-// inside the domain and their list: the others are zero in the result and no
-// sum is formed for them (blocks past the number return at once).
-// 350^2 points of a star's bounding square on its 16,384 nodes, test and
-// sums: 1.94 ms -> 0.83 ms, the sums about five sixths of it.
-constexpr int kDomPair = kDomThreads / 2;
-template <int PDE>
-__global__ void __launch_bounds__(kDomPair)
+// A thread owns H targets of a block's 256 (two, 128 apart, where the blocks
+// fill the GPU), as in the operator product: bound by the FP64 pipe.  live,
+// if given, is the number of points inside the domain and their list: the
+// others are zero in the result and no sum is formed for them (blocks past
+// the number return at once).  350^2 points of a star's bounding square on
+// its 16,384 nodes, test and sums: 1.94 ms -> 0.83 ms, the sums about five
+// sixths of it.
+template <int PDE, int H>
+__global__ void __launch_bounds__(kDomThreads / H)
     domain_partial_kernel(const Node* __restrict__ nodes, int np, int nt,
                           const double* __restrict__ tg, const int* __restrict__ live,
                           const double* __restrict__ mu, int chunk, long long stride,
                           double* __restrict__ part) {
   const int count = live ? live[0] : nt;
   if (blockIdx.x * kDomThreads >= count) return;
-  __shared__ double2 spos[kDomThreads], samp[kDomThreads], sden[kDomThreads];
-  int t[2];
-  double tx[2], ty[2], y0[2] = {0.0, 0.0}, y1[2] = {0.0, 0.0};
+  constexpr int T = kDomThreads / H;
+  __shared__ SourceArray<(H > 1), kDomThreads> spos, samp, sden;
+  int t[H];
+  double tx[H], ty[H], y0[H], y1[H];
 #pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const int i = blockIdx.x * kDomThreads + threadIdx.x + h * kDomPair;
+  for (int h = 0; h < H; h++) {
+    const int i = blockIdx.x * kDomThreads + threadIdx.x + h * T;
     t[h] = i < count ? (live ? live[1 + i] : i) : -1;
     tx[h] = t[h] >= 0 ? tg[2 * t[h]] : 0.0;
     ty[h] = t[h] >= 0 ? tg[2 * t[h] + 1] : 0.0;
+    y0[h] = y1[h] = 0.0;
   }
   const int s0 = blockIdx.y * chunk;
   const int s1 = min(np, s0 + chunk);
   for (int base = s0; base < s1; base += kDomThreads) {
     __syncthreads();
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int k = threadIdx.x + h * kDomPair, j = base + k;
+    for (int h = 0; h < H; h++) {
+      const int k = threadIdx.x + h * T, j = base + k;
       if (j < s1) {
         const Node s = nodes[j];
-        spos[k] = make_double2(s.x, s.y);
+        spos.put(k, s.x, s.y);
         if (PDE == kLaplace) {
           const double c = -s.w * KI_INV_2PI * mu[j];
-          samp[k] = make_double2(c * s.nx, c * s.ny);
+          samp.put(k, c * s.nx, c * s.ny);
         } else if (PDE == kLaplaceNeumann) {
-          samp[k] = make_double2(s.w * KI_INV_2PI * mu[j], 0.0);
+          samp.put(k, s.w * KI_INV_2PI * mu[j], 0.0);
         } else {
           const double c = s.w * KI_INV_PI;
-          samp[k] = make_double2(c * s.nx, c * s.ny);
-          sden[k] = make_double2(mu[2 * j], mu[2 * j + 1]);
+          samp.put(k, c * s.nx, c * s.ny);
+          sden.put(k, mu[2 * j], mu[2 * j + 1]);
         }
       } else {
         // padding: a far source of zero strength (|r|^2 stays inside the
         // range of the reciprocal estimate; every numerator is zero)
-        spos[k] = make_double2(1e15, 1e15);
-        samp[k] = sden[k] = make_double2(0.0, 0.0);
+        spos.put(k, 1e15, 1e15);
+        samp.put(k, 0.0, 0.0);
+        sden.put(k, 0.0, 0.0);
       }
     }
     __syncthreads();
 #pragma unroll 4
     for (int q = 0; q < kDomThreads; q++) {
-      const double2 p = spos[q], a = samp[q];
-      const double2 d = PDE == kStokes ? sden[q] : make_double2(0.0, 0.0);
+      const double2 p = spos.get(q), a = samp.get(q);
+      const double2 d = PDE == kStokes ? sden.get(q) : make_double2(0.0, 0.0);
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
+      for (int h = 0; h < H; h++) {
         if (PDE == kLaplaceNeumann) {
           const double r0 = tx[h] - p.x, r1 = ty[h] - p.y;
           y0[h] += a.x * (0.5 * log(r0 * r0 + r1 * r1));
@@ -105,7 +108,7 @@ __global__ void __launch_bounds__(kDomPair)
     }
   }
 #pragma unroll
-  for (int h = 0; h < 2; h++) {
+  for (int h = 0; h < H; h++) {
     if (t[h] < 0) continue;
     if (PDE == kStokes) {
       part[stride * blockIdx.y + 2 * t[h]] = y0[h];
@@ -398,11 +401,29 @@ cudaError_t launch_domain_mask(int kind, const Node* nodes, int np, const double
   return cudaGetLastError();
 }
 
+namespace {
+template <int H>
+void launch_partial(int pde, dim3 grid, const Node* nodes, int np, int nt, const double* targets,
+                    const int* inside, const double* mu, int chunk, long long rows, double* dst,
+                    cudaStream_t s) {
+  constexpr int T = kDomThreads / H;
+  if (pde == kLaplace)
+    domain_partial_kernel<kLaplace, H><<<grid, T, 0, s>>>(nodes, np, nt, targets, inside, mu,
+                                                          chunk, rows, dst);
+  else if (pde == kLaplaceNeumann)
+    domain_partial_kernel<kLaplaceNeumann, H><<<grid, T, 0, s>>>(nodes, np, nt, targets, inside,
+                                                                mu, chunk, rows, dst);
+  else
+    domain_partial_kernel<kStokes, H><<<grid, T, 0, s>>>(nodes, np, nt, targets, inside, mu,
+                                                         chunk, rows, dst);
+}
+}  // namespace
+
 cudaError_t launch_domain_eval(int pde, const Node* nodes, int np, int nt,
                                const double* targets, const double* mu, int nh,
                                const double* holes, const double* alpha,
                                const unsigned char* mask, const int* inside, int splits,
-                               double* part, double* out, cudaStream_t s) {
+                               double* part, double* out, int num_sms, cudaStream_t s) {
   if (nt == 0) return cudaSuccess;
   const int sd = pde == kStokes ? 2 : 1;
   const long long rows = static_cast<long long>(nt) * sd;
@@ -410,15 +431,10 @@ cudaError_t launch_domain_eval(int pde, const Node* nodes, int np, int nt,
   const int chunk = (np + splits - 1) / splits;
   const dim3 grid((nt + kDomThreads - 1) / kDomThreads, splits);
   count_launches(2);
-  if (pde == kLaplace) {
-    domain_partial_kernel<kLaplace><<<grid, kDomPair, 0, s>>>(nodes, np, nt, targets, inside, mu,
-                                                              chunk, rows, dst);
-  } else if (pde == kLaplaceNeumann) {
-    domain_partial_kernel<kLaplaceNeumann><<<grid, kDomPair, 0, s>>>(nodes, np, nt, targets,
-                                                                    inside, mu, chunk, rows, dst);
+  if (sum_targets(static_cast<long long>(grid.x) * splits, num_sms) == 1) {
+    launch_partial<1>(pde, grid, nodes, np, nt, targets, inside, mu, chunk, rows, dst, s);
   } else {
-    domain_partial_kernel<kStokes><<<grid, kDomPair, 0, s>>>(nodes, np, nt, targets, inside, mu,
-                                                             chunk, rows, dst);
+    launch_partial<2>(pde, grid, nodes, np, nt, targets, inside, mu, chunk, rows, dst, s);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;

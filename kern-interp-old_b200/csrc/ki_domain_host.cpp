@@ -69,7 +69,7 @@ int Solver::eval_domain(int nt, const double* d_targets, const double* d_mu,
   const bool use_alpha = nb_ > 0 && d_alpha;
   KI_CUDA(launch_domain_eval(opt_.pde, d_nodes_, n_points_, nt, d_targets, d_mu, n_holes(),
                              d_holes_, use_alpha ? d_alpha : nullptr, mask, inside, splits, part,
-                             d_out, stream_));
+                             d_out, num_sms_, stream_));
   return 0;
 }
 

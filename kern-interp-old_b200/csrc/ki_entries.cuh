@@ -57,6 +57,27 @@ __device__ __forceinline__ double rcp_dist2(double rr) {
   return __double2hiint(rr) != 0 ? nr_rcp(rr) : 0.0;
 }
 
+// Two values of each of N sources of the FP64 operator and domain sums, in
+// shared memory.  PAIRED: read as 16-byte pairs, half the loads, for kernels
+// with two targets a thread on a full GPU; else as 8-byte values, which
+// arrive sooner: with few warps a source's loads are waited for (200 Laplace
+// nodes at one point: 19.2 us in pairs, 16.3 us).
+template <bool PAIRED, int N>
+struct SourceArray {
+  double2 v[N];
+  __device__ __forceinline__ void put(int k, double a, double b) { v[k] = make_double2(a, b); }
+  __device__ __forceinline__ double2 get(int k) const { return v[k]; }
+};
+template <int N>
+struct SourceArray<false, N> {
+  double x[N], y[N];
+  __device__ __forceinline__ void put(int k, double a, double b) {
+    x[k] = a;
+    y[k] = b;
+  }
+  __device__ __forceinline__ double2 get(int k) const { return make_double2(x[k], y[k]); }
+};
+
 // One pair of the FP64 operator and domain sums: source at (sx, sy) with the
 // staged values a0, a1 (and density d0, d1 for Stokes), target at (tx, ty)
 // with normal (tnx, tny) (Laplace-Neumann), added to y0, y1.  Stokes: 17 FP64

@@ -373,7 +373,7 @@ cudaError_t launch_domain_eval(int pde, const Node* nodes, int np, int nt,
                                const double* targets, const double* mu, int nh,
                                const double* holes, const double* alpha,
                                const unsigned char* mask, const int* inside, int splits,
-                               double* part, double* out, cudaStream_t s);
+                               double* part, double* out, int num_sms, cudaStream_t s);
 // cudaFuncSetAttribute(func, attr, value) unless this process already
 // raised the attribute to at least `value` on the current device: the call
 // costs microseconds of host time, which level loops with many short
@@ -420,6 +420,14 @@ struct MvTile {
 // whose tiles fill whole waves of the resident CTAs best (a last, partly
 // filled wave costs as much time as a full one).
 int matvec_splits(int pde, int n_nodes, int nseg, int num_sms);
+// Targets per thread of the FP64 operator and domain sums, by the 256-target
+// blocks of a launch.  Two keep a full GPU's FP64 pipe busier (16,384 Laplace
+// nodes, 28 blocks per SM: 218 us, one 226 us), but halve the warps of a
+// launch that does not fill it (1,000 nodes: 21 us, one 17 us; 3,000 nodes at
+// 30,000 points, 5 per SM: 97 us, one 88 us; even between 8 and 15 per SM).
+inline int sum_targets(long long blocks, int num_sms) {
+  return blocks > 8LL * num_sms ? 2 : 1;
+}
 // seg: node offsets of the segments (size nseg + 1); one segment = one
 // problem, so a forest's operator is block diagonal.
 void matvec_tiles(const std::vector<int>& seg, int splits, std::vector<MvTile>* tiles);
@@ -427,7 +435,7 @@ size_t fast_matvec_scratch_doubles(int n_dofs, int splits, int nseg, int nb);
 cudaError_t launch_fast_matvec(int pde, const Node* nodes, const MvTile* tiles, int ntiles,
                                const int* seg, int nseg, int n_dofs, int splits, const double* x,
                                double* y, int nb, const double* U, const double* Psi,
-                               double* part, cudaStream_t s);
+                               double* part, int num_sms, cudaStream_t s);
 // The same product for a small correction d (see ki_krylov.cu): source
 // blocks whose bounding box comes within near_gap of the target tile's in
 // FP64, the others in FP32 with the densities scaled by dscale (> 0).

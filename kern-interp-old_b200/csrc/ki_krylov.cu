@@ -9,7 +9,7 @@
 //     pass, several axpys in one pass, scaling), all with a fixed reduction
 //     order so a solve is reproducible.
 //
-// Operator product layout: two target nodes per thread, 256 targets per CTA,
+// Operator product layout: 256 targets per CTA, one or two per thread,
 // sources staged 256 at a time in shared memory as structure-of-arrays with
 // the density folded in; the source range is split over gridDim.y so the
 // grid covers every SM, and the splits' partial sums are added in order by
@@ -29,28 +29,28 @@ constexpr int kMvThreads = 256;
 //   Laplace:          a = -(w / 2 pi) x (n_x, n_y)
 //   Laplace-Neumann:  a = (w / 2 pi) x (1, 1)      (target normal applied later)
 //   Stokes:           a = (w / pi) (n_x, n_y), density (x0, x1)
-// A thread owns two targets of the 256-target tile, t and t + 128: a source's
-// values are loaded from shared memory once for both, as 16-byte loads, and
-// two independent chains per source keep the FP64 pipe, which bounds this
-// kernel, full.  65,536 Stokes dofs: 1.31 ms -> 1.17 ms with the two targets
-// and the zero test off that pipe; the pipe's own time for 17 operations per
-// pair is 1.14 ms (one warp instruction in 2.25 cycles per scheduler).
-constexpr int kPairThreads = kMvThreads / 2;
-
-template <int PDE>
-__global__ void __launch_bounds__(kPairThreads)
+// A thread owns H targets of the 256-target tile.  Two, t and t + 128, where
+// the blocks fill the GPU: a source's values are loaded from shared memory
+// once for both, as 16-byte loads, and two independent chains per source keep
+// the FP64 pipe, which bounds this kernel, full.  65,536 Stokes dofs: 1.31 ms
+// -> 1.17 ms with the two targets and the zero test off that pipe; the pipe's
+// own time for 17 operations per pair is 1.10 ms (one warp instruction in
+// 2.25 cycles per scheduler).
+template <int PDE, int H>
+__global__ void __launch_bounds__(kMvThreads / H)
     mv_partial_kernel(const Node* __restrict__ nodes, const MvTile* __restrict__ tiles,
                       long long part_stride, const double* __restrict__ x,
                       double* __restrict__ part, double* __restrict__ part_rank1) {
-  __shared__ double2 spos[kMvThreads], samp[kMvThreads], sden[kMvThreads];
-  __shared__ double red[kPairThreads / 32];
+  constexpr int T = kMvThreads / H;
+  __shared__ SourceArray<(H > 1), kMvThreads> spos, samp, sden;
+  __shared__ double red[T / 32];
   const MvTile tile = tiles[blockIdx.x];
   const int s0 = tile.s0, s1 = tile.s1;
-  double tx[2], ty[2], tnx[2], tny[2], y0[2] = {0.0, 0.0}, y1[2] = {0.0, 0.0}, r1 = 0.0;
+  double tx[H], ty[H], tnx[H], tny[H], y0[H], y1[H], r1 = 0.0;
 #pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const int t = tile.t0 + threadIdx.x + h * kPairThreads;
-    tx[h] = ty[h] = tnx[h] = tny[h] = 0.0;
+  for (int h = 0; h < H; h++) {
+    const int t = tile.t0 + threadIdx.x + h * T;
+    tx[h] = ty[h] = tnx[h] = tny[h] = y0[h] = y1[h] = 0.0;
     if (t < tile.t1) {
       const Node nt = nodes[t];
       tx[h] = nt.x;
@@ -62,46 +62,47 @@ __global__ void __launch_bounds__(kPairThreads)
   for (int base = s0; base < s1; base += kMvThreads) {
     __syncthreads();
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int k = threadIdx.x + h * kPairThreads, j = base + k;
+    for (int h = 0; h < H; h++) {
+      const int k = threadIdx.x + h * T, j = base + k;
       if (j < s1) {
         const Node s = nodes[j];
-        spos[k] = make_double2(s.x, s.y);
+        spos.put(k, s.x, s.y);
         if (PDE == kLaplace) {
           const double c = -s.w * KI_INV_2PI * x[j];
-          samp[k] = make_double2(c * s.nx, c * s.ny);
+          samp.put(k, c * s.nx, c * s.ny);
         } else if (PDE == kLaplaceNeumann) {
-          samp[k] = make_double2(s.w * KI_INV_2PI * x[j], 0.0);
+          samp.put(k, s.w * KI_INV_2PI * x[j], 0.0);
           // rank-one part: sum_j w_j x_j (the "+ w_s" of every entry)
           if (tile.first) r1 += s.w * x[j];
         } else {
           const double c = s.w * KI_INV_PI;
-          samp[k] = make_double2(c * s.nx, c * s.ny);
+          samp.put(k, c * s.nx, c * s.ny);
           const double d0 = x[2 * j], d1 = x[2 * j + 1];
-          sden[k] = make_double2(d0, d1);
+          sden.put(k, d0, d1);
           // rank-one part: sum_j w_j (n_j . x_j), applied as tn_t * sum
           if (tile.first) r1 += s.w * (s.nx * d0 + s.ny * d1);
         }
       } else {
         // padding: a source far away with zero strength (|r|^2 stays within
         // the range of the reciprocal estimate; its numerators are zero)
-        spos[k] = make_double2(1e15, 1e15);
-        samp[k] = sden[k] = make_double2(0.0, 0.0);
+        spos.put(k, 1e15, 1e15);
+        samp.put(k, 0.0, 0.0);
+        sden.put(k, 0.0, 0.0);
       }
     }
     __syncthreads();
 #pragma unroll 4
     for (int q = 0; q < kMvThreads; q++) {
-      const double2 p = spos[q], a = samp[q];
-      const double2 d = PDE == kStokes ? sden[q] : make_double2(0.0, 0.0);
+      const double2 p = spos.get(q), a = samp.get(q);
+      const double2 d = PDE == kStokes ? sden.get(q) : make_double2(0.0, 0.0);
 #pragma unroll
-      for (int h = 0; h < 2; h++)
+      for (int h = 0; h < H; h++)
         pair_sum<PDE>(tx[h], ty[h], tnx[h], tny[h], p.x, p.y, a.x, a.y, d.x, d.y, y0[h], y1[h]);
     }
   }
 #pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const int t = tile.t0 + threadIdx.x + h * kPairThreads;
+  for (int h = 0; h < H; h++) {
+    const int t = tile.t0 + threadIdx.x + h * T;
     if (t >= tile.t1) continue;
     if (PDE == kStokes) {
       part[part_stride * tile.split + 2 * t] = y0[h];
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(kPairThreads)
     __syncthreads();
     if (threadIdx.x == 0) {
       double v = 0.0;
-      for (int w = 0; w < kPairThreads / 32; w++) v += red[w];
+      for (int w = 0; w < T / 32; w++) v += red[w];
       part_rank1[tile.rank1_slot] = v;
     }
   }
@@ -554,11 +555,13 @@ __global__ void segment_sumsq_kernel(const double* __restrict__ v, const int* __
 int matvec_splits(int pde, int n_nodes, int nseg, int num_sms) {
   // resident CTAs of the product kernel on the whole GPU
   int per_sm = 0;
-  const void* fn = pde == kLaplace ? reinterpret_cast<const void*>(&mv_partial_kernel<kLaplace>)
+  const void* fn = pde == kLaplace
+                       ? reinterpret_cast<const void*>(&mv_partial_kernel<kLaplace, 2>)
                    : pde == kLaplaceNeumann
-                       ? reinterpret_cast<const void*>(&mv_partial_kernel<kLaplaceNeumann>)
-                       : reinterpret_cast<const void*>(&mv_partial_kernel<kStokes>);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPairThreads, 0) != cudaSuccess ||
+                       ? reinterpret_cast<const void*>(&mv_partial_kernel<kLaplaceNeumann, 2>)
+                       : reinterpret_cast<const void*>(&mv_partial_kernel<kStokes, 2>);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kMvThreads / 2, 0) !=
+          cudaSuccess ||
       per_sm < 1)
     per_sm = 1;
   const long long slots = static_cast<long long>(per_sm) * std::max(1, num_sms);
@@ -595,22 +598,33 @@ void matvec_tiles(const std::vector<int>& seg, int splits, std::vector<MvTile>* 
   }
 }
 
+namespace {
+template <int H>
+void launch_partial(int pde, const Node* nodes, const MvTile* tiles, int ntiles, int n_dofs,
+                    const double* x, double* part, double* part_rank1, cudaStream_t s) {
+  constexpr int T = kMvThreads / H;
+  if (pde == kLaplace)
+    mv_partial_kernel<kLaplace, H><<<ntiles, T, 0, s>>>(nodes, tiles, n_dofs, x, part, part_rank1);
+  else if (pde == kLaplaceNeumann)
+    mv_partial_kernel<kLaplaceNeumann, H><<<ntiles, T, 0, s>>>(nodes, tiles, n_dofs, x, part,
+                                                              part_rank1);
+  else
+    mv_partial_kernel<kStokes, H><<<ntiles, T, 0, s>>>(nodes, tiles, n_dofs, x, part, part_rank1);
+}
+}  // namespace
+
 cudaError_t launch_fast_matvec(int pde, const Node* nodes, const MvTile* tiles, int ntiles,
                                const int* seg, int nseg, int n_dofs, int splits, const double* x,
                                double* y, int nb, const double* U, const double* Psi,
-                               double* part, cudaStream_t s) {
+                               double* part, int num_sms, cudaStream_t s) {
   if (splits < 1 || splits > kMaxMatvecSplits) return cudaErrorInvalidValue;
   double* part_rank1 = part + static_cast<long long>(splits) * n_dofs;
   count_launches(nb ? 3 : 2);
-  if (pde == kLaplace)
-    mv_partial_kernel<kLaplace><<<ntiles, kPairThreads, 0, s>>>(nodes, tiles, n_dofs, x, part,
-                                                               part_rank1);
-  else if (pde == kLaplaceNeumann)
-    mv_partial_kernel<kLaplaceNeumann><<<ntiles, kPairThreads, 0, s>>>(nodes, tiles, n_dofs, x,
-                                                                      part, part_rank1);
-  else
-    mv_partial_kernel<kStokes><<<ntiles, kPairThreads, 0, s>>>(nodes, tiles, n_dofs, x, part,
-                                                              part_rank1);
+  if (sum_targets(ntiles, num_sms) == 1) {
+    launch_partial<1>(pde, nodes, tiles, ntiles, n_dofs, x, part, part_rank1, s);
+  } else {
+    launch_partial<2>(pde, nodes, tiles, ntiles, n_dofs, x, part, part_rank1, s);
+  }
   mv_finish_kernel<<<(n_dofs + 255) / 256, 256, 0, s>>>(pde, nodes, n_dofs, splits, part,
                                                         part_rank1, seg, nseg, x, y, nb, U);
   if (nb) {

@@ -101,7 +101,7 @@ int Solver::matvec_device(const double* d_x, double* d_y) {
   if (kry_.bytes < sizeof(double) * need) KI_CUDA(kry_.reserve(sizeof(double) * need, stream_));
   KI_CUDA(launch_fast_matvec(opt_.pde, d_nodes_, d_mv_tiles_, n_mv_tiles_, d_seg_, nseg, n_dofs_,
                              mv_splits_, d_x, d_y, nb_, d_U_, d_Psi_, static_cast<double*>(kry_.p),
-                             stream_));
+                             num_sms_, stream_));
   return 0;
 }
 
