@@ -428,7 +428,8 @@ cudaError_t launch_domain_eval(int pde, const Node* nodes, int np, int nt,
   const int sd = pde == kStokes ? 2 : 1;
   const long long rows = static_cast<long long>(nt) * sd;
   double* dst = splits > 1 ? part : out;
-  const int chunk = (np + splits - 1) / splits;
+  // (whole tiles of sources: 700 in two chunks are three tiles, not four)
+  const int chunk = ((np + splits - 1) / splits + kDomThreads - 1) / kDomThreads * kDomThreads;
   const dim3 grid((nt + kDomThreads - 1) / kDomThreads, splits);
   count_launches(2);
   if (sum_targets(static_cast<long long>(grid.x) * splits, num_sms) == 1) {
