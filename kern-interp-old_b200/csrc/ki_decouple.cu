@@ -228,7 +228,10 @@ __host__ __device__ inline DecLayout dec_layout(int n, int k, bool tl) {
 }
 
 // FAST: entries by contracted arithmetic (a preconditioner's, whose sketched
-// IDs use it too); else the reference's bits, and L corrected.  TL: T is
+// IDs use it too: on stars and circles of 1,024 to 32,768 nodes their rms
+// error against 64-bit significands is 0.57 to 0.92 of that of the reference's
+// order of roundings, for every kernel and distance); else the reference's
+// bits, and L corrected.  TL: T is
 // copied to shared memory, where L takes its place; else, for boxes whose
 // K_BN leaves no room for it (149 dofs and more, by rank), the products read
 // T, and L as it is made, in global memory (from L1: a warp's fragment is

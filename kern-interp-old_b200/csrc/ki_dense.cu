@@ -1731,7 +1731,11 @@ cudaError_t launch_border_rhs(const double* Pred, int nr, int nb, const double* 
 // w - (X^{-1} U) alpha, with X^{-1} w in x already and X^{-1} U kept by the
 // factorization, so that the diagonal blocks are read once a solve (of eight
 // holes and 65,536 dofs: this kernel and the two above 19 us, the products,
-// gathers and second diagonal solve they replace 73 us).
+// gathers and second diagonal solve they replace 73 us).  The difference is
+// taken after X^{-1}: where w and U alpha nearly agree it could lose digits.
+// Measured with w = U alpha on 15 domains of 1 to 8 holes, 300 to 1,500
+// nodes, against extended precision: 0.1 to 4.2 times the error of X^{-1} (w
+// - U alpha) in single solves, 0.8 (id_tol 1e-10) and 0.5 (1e-15) in the mean.
 __global__ void __launch_bounds__(kBorderThreads)
     border_apply_kernel(const double* __restrict__ dinv, int nr, int nb,
                         const int* __restrict__ allred, const int* __restrict__ allskel, int ns,

@@ -613,10 +613,15 @@ __device__ __forceinline__ void oc_tsolve(int k, int n, int g, int G, const int*
 // them is taken as LAPACK takes the first of equal ones: a column's entries
 // err by about eps |A|, its squared norm relatively by 2 eps |A| / norm, so
 // the key drops 4 bits plus half the bits the squared norm has lost since
-// the start (e0: exponent of the largest).  On mirror-symmetric boundaries
-// the choice among tied columns then hardly depends on the order of the
-// sums; 8 bits would merge columns that do differ (on some eight-hole Stokes
-// domains, up to 8 of 1,500 skeletons; none with 4 bits).
+// the start (e0: exponent of the largest): columns whose squares differ by
+// less than 4e-15, late in a box at id_tol 1e-10 by less than 3e-5, both
+// about 16 times their rounding error.  Tied columns are then usually, not
+// always, taken by position: two on either side of a step of the key are
+// not.  Against the CPU restatement of LAPACK's steps, 24 eight-hole Stokes
+// domains (16,384 dofs, 13,272 boxes, id_tol 1e-10): 30 boxes in 5 domains
+// differ, with the exact comparison 33 in 4 (equally spaced nodes on the
+// holes tie); ellipses and stars (6,957 boxes): none by either.  Sketched
+// boxes, and id_kernel with its boxes past shared memory, compare exactly.
 __device__ __forceinline__ unsigned long long oc_cand_key(double v, int e0, bool sketched) {
   if (!(v > 0.0)) return 0ull;
   const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v));

@@ -82,7 +82,7 @@ struct IdParams {
 // with G CTAs per box; kTile + 100 t + G keeps the matrix or its row sketch
 // (IdTask::sk rows) in the registers of a G-CTA cluster, tile shape t;
 // kOnChip + G (G = 1 .. 16) keeps the matrix in the cluster's shared memory,
-// kSketched + G (G = 8, 16) the sketch, kSpilled + G (G = 8, 16) the first
+// kSketched + G (G = 1, 2, 8, 16) the sketch, kSpilled + G (G = 8, 16) the first
 // IdTask::nres columns, the others in the workspace.
 constexpr int kOnChip = 100, kSketched = 200, kSpilled = 300, kTile = 1000;
 // Rows of an on-chip ID matrix over a G-CTA cluster: every CTA gets the same

@@ -112,7 +112,8 @@ __device__ __forceinline__ void apply_sub_multi(double* out, const double* in, i
 // global memory: each box is swept by a cluster of kWideCluster CTAs, which
 // deal the rows of a product among themselves (a single SM's loads, and not
 // the HBM, would bound a box on one CTA).  The rows [r0, r0 + cnt) of CTA g,
-// whole 32-byte sectors:
+// four at a time (whole 32-byte sectors where the leading dimension is a
+// multiple of four):
 constexpr int kWideThreads = 512;
 constexpr int kWideCluster = 8;
 __device__ __forceinline__ void wide_rows(int rows, int g, int* r0, int* cnt) {
