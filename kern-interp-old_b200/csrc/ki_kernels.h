@@ -416,10 +416,13 @@ constexpr int kMaxKrylov = 64;  // vectors per multi-dot
 struct MvTile {
   int t0, t1, s0, s1, split, rank1_slot, first, pad;
 };
-// Source splits for nseg segments of about n_nodes nodes each: the count
-// whose tiles fill whole waves of the resident CTAs best (a last, partly
-// filled wave costs as much time as a full one).
-int matvec_splits(int pde, int n_nodes, int nseg, int num_sms);
+// Source splits of the segments [seg[p], seg[p + 1]).  One: the count whose
+// tiles fill whole waves of the resident CTAs best (a last, partly filled wave
+// costs as much time as a full one).  Several, of uneven sizes, come without
+// waves: the count of the least time by Graham's bound, all blocks' work over
+// the resident CTAs plus the longest block (64 problems of 512 to 8,192 nodes:
+// 711 us; 806 us by the rule above at their mean size).
+int matvec_splits(int pde, const std::vector<int>& seg, int num_sms);
 // Targets per thread of the FP64 operator and domain sums, by the 256-target
 // blocks of a launch.  Two keep a full GPU's FP64 pipe busier (16,384 Laplace
 // nodes, 28 blocks per SM: 218 us, one 226 us), but halve the warps of a

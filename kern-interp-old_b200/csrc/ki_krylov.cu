@@ -552,7 +552,7 @@ __global__ void segment_sumsq_kernel(const double* __restrict__ v, const int* __
 
 }  // namespace
 
-int matvec_splits(int pde, int n_nodes, int nseg, int num_sms) {
+int matvec_splits(int pde, const std::vector<int>& seg, int num_sms) {
   // resident CTAs of the product kernel on the whole GPU
   int per_sm = 0;
   const void* fn = pde == kLaplace
@@ -565,14 +565,27 @@ int matvec_splits(int pde, int n_nodes, int nseg, int num_sms) {
       per_sm < 1)
     per_sm = 1;
   const long long slots = static_cast<long long>(per_sm) * std::max(1, num_sms);
-  const int per_seg = (n_nodes + kMvThreads - 1) / kMvThreads;  // target tiles
-  const long long tblocks = static_cast<long long>(per_seg) * std::max(1, nseg);
-  const int max_split = std::max(1, std::min(per_seg, kMaxMatvecSplits));  // >= 256 sources each
-  // time ~ waves x (sources per split): minimise ceil(tblocks S / slots) / S
+  std::vector<int> tiles;  // 256-node tiles of each segment
+  int most = 1;
+  for (size_t p = 0; p + 1 < seg.size(); p++) {
+    tiles.push_back((seg[p + 1] - seg[p] + kMvThreads - 1) / kMvThreads);
+    most = std::max(most, tiles.back());
+  }
+  const bool one = tiles.size() == 1;
   int best = 1;
   double best_t = 1e300;
-  for (int S = 1; S <= max_split; S++) {
-    const double t = static_cast<double>((tblocks * S + slots - 1) / slots) / S;
+  for (int S = 1; S <= std::min(most, kMaxMatvecSplits); S++) {  // >= 256 sources each
+    double t;
+    if (one) {
+      // ~ waves x (sources per split): ceil(blocks / slots) / S
+      const long long blocks = static_cast<long long>(most) * S;
+      t = static_cast<double>((blocks + slots - 1) / slots) / S;
+    } else {
+      // in source tiles; a block itself costs about a third of one
+      double work = 0.0;
+      for (int n : tiles) work += n * (n + S / 3.0);
+      t = work / slots + (most + S - 1) / S + 1.0 / 3.0;
+    }
     if (t < best_t * (1.0 - 1e-9)) {
       best_t = t;
       best = S;

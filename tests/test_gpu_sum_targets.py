@@ -38,3 +38,18 @@ def test_domain(pde, nt):
     tg = np.random.default_rng(1).uniform(-1.5, 1.5, 2 * nt)
     out, exact = s.eval_domain(tg, mu, al, "all"), s.eval_targets(tg, mu, al)
     assert np.abs(out - exact).max() <= 8 * 2.0**-53 * s.n_dofs * np.abs(exact).max()
+
+
+@pytest.mark.parametrize("sizes", [(17, 300, 257, 6000), (256, 256), (512, 700, 8192)])
+def test_operator_of_uneven_problems(sizes):
+    """More source splits than a small problem has tiles: the rest are empty."""
+    import torch
+    rng = np.random.default_rng(sizes[0])
+    b = kinterp.BatchSolver([G.random_star(rng, n, 64) for n in sizes], id_tol=1e-3)
+    x = torch.tensor(rng.standard_normal(b.n_dofs), device="cuda")
+    y, z = torch.empty_like(x), torch.empty_like(x)
+    b.apply_device(x.data_ptr(), y.data_ptr())
+    kinterp.Solver.matvec_device(b, x.data_ptr(), z.data_ptr())
+    torch.cuda.synchronize()
+    for n, p, q in zip(sizes, b.split(y), b.split(z)):
+        assert (p - q).abs().max() <= 8 * 2.0**-53 * n * p.abs().max()
