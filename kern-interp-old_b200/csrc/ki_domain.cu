@@ -41,7 +41,7 @@ constexpr double kDomainEps = 1e-2;  // cubic_boundary.cpp:185, circle.cpp:37
 // if given, is the number of points inside the domain and their list: the
 // others are zero in the result and no sum is formed for them (blocks past
 // the number return at once).  350^2 points of a star's bounding square on
-// its 16,384 nodes, test and sums: 1.94 ms -> 0.83 ms, the sums about five
+// its 16,384 nodes, test and sums: 1.94 ms -> 0.76 ms, the sums about five
 // sixths of it.
 template <int PDE, int H>
 __global__ void __launch_bounds__(kDomThreads / H)
@@ -92,17 +92,21 @@ __global__ void __launch_bounds__(kDomThreads / H)
       }
     }
     __syncthreads();
-#pragma unroll 4
-    for (int q = 0; q < kDomThreads; q++) {
-      const double2 p = spos.get(q), a = samp.get(q);
-      const double2 d = PDE == kStokes ? sden.get(q) : make_double2(0.0, 0.0);
+    const int cnt = min(kDomThreads, (s1 - base + 3) & ~3);  // (the padding past it is not summed)
+#pragma unroll 1
+    for (int q4 = 0; q4 < cnt; q4 += 4) {
 #pragma unroll
-      for (int h = 0; h < H; h++) {
-        if (PDE == kLaplaceNeumann) {
-          const double r0 = tx[h] - p.x, r1 = ty[h] - p.y;
-          y0[h] += a.x * (0.5 * log(r0 * r0 + r1 * r1));
-        } else {
-          pair_sum<PDE>(tx[h], ty[h], 0.0, 0.0, p.x, p.y, a.x, a.y, d.x, d.y, y0[h], y1[h]);
+      for (int q = q4; q < q4 + 4; q++) {
+        const double2 p = spos.get(q), a = samp.get(q);
+        const double2 d = PDE == kStokes ? sden.get(q) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+          if (PDE == kLaplaceNeumann) {
+            const double r0 = tx[h] - p.x, r1 = ty[h] - p.y;
+            y0[h] += a.x * (0.5 * log(r0 * r0 + r1 * r1));
+          } else {
+            pair_sum<PDE>(tx[h], ty[h], 0.0, 0.0, p.x, p.y, a.x, a.y, d.x, d.y, y0[h], y1[h]);
+          }
         }
       }
     }
@@ -432,7 +436,7 @@ cudaError_t launch_domain_eval(int pde, const Node* nodes, int np, int nt,
   const int chunk = ((np + splits - 1) / splits + kDomThreads - 1) / kDomThreads * kDomThreads;
   const dim3 grid((nt + kDomThreads - 1) / kDomThreads, splits);
   count_launches(2);
-  if (sum_targets(static_cast<long long>(grid.x) * splits, num_sms) == 1) {
+  if (sum_targets(static_cast<long long>(grid.x) * splits, num_sms, kDomainSingle) == 1) {
     launch_partial<1>(pde, grid, nodes, np, nt, targets, inside, mu, chunk, rows, dst, s);
   } else {
     launch_partial<2>(pde, grid, nodes, np, nt, targets, inside, mu, chunk, rows, dst, s);

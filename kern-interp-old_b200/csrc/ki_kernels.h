@@ -416,20 +416,24 @@ constexpr int kMaxKrylov = 64;  // vectors per multi-dot
 struct MvTile {
   int t0, t1, s0, s1, split, rank1_slot, first, pad;
 };
-// Source splits of the segments [seg[p], seg[p + 1]).  One: the count whose
-// tiles fill whole waves of the resident CTAs best (a last, partly filled wave
-// costs as much time as a full one).  Several, of uneven sizes, come without
-// waves: the count of the least time by Graham's bound, all blocks' work over
-// the resident CTAs plus the longest block (64 problems of 512 to 8,192 nodes:
-// 711 us; 806 us by the rule above at their mean size).
+// Source splits of the segments [seg[p], seg[p + 1]): the count of the least
+// time by Graham's bound, all blocks' work over the resident CTAs plus the
+// longest block.  Counts whose blocks fill whole waves, the former rule, lose
+// where sizes are uneven and where whole tiles make the splits so: 64 problems
+// of 512 to 8,192 nodes 806 -> 711 us, 21,000 Stokes nodes 544 -> 528 us, 9,000
+// Laplace nodes 111 -> 87 us.
 int matvec_splits(int pde, const std::vector<int>& seg, int num_sms);
 // Targets per thread of the FP64 operator and domain sums, by the 256-target
-// blocks of a launch.  Two keep a full GPU's FP64 pipe busier (16,384 Laplace
-// nodes, 28 blocks per SM: 218 us, one 226 us), but halve the warps of a
-// launch that does not fill it (1,000 nodes: 21 us, one 17 us; 3,000 nodes at
-// 30,000 points, 5 per SM: 97 us, one 88 us; even between 8 and 15 per SM).
-inline int sum_targets(long long blocks, int num_sms) {
-  return blocks > 8LL * num_sms ? 2 : 1;
+// blocks of a launch: one up to one block per SM (domain sums: two), else two.
+// Two keep the FP64 pipe of a full GPU busier, but halve the warps of a block
+// (operator, 2,500 Laplace nodes, 100 blocks: one 27.7 us alone and 7.7 us
+// among others, two 32.1 and 7.8; 4,096 nodes, 256 blocks: 32.8 and 13.2, two
+// 33.0 and 12.7.  19,600 points at 1,000 nodes, 154 blocks: 47.2 and 15.4,
+// two 68.1 and 19.1; 2,809 at 16,384 nodes, 352 blocks: 67.6 and 35.0, two
+// 79.6 and 34.0).
+constexpr int kOperatorSingle = 1, kDomainSingle = 2;
+inline int sum_targets(long long blocks, int num_sms, int single) {
+  return blocks > static_cast<long long>(single) * num_sms ? 2 : 1;
 }
 // seg: node offsets of the segments (size nseg + 1); one segment = one
 // problem, so a forest's operator is block diagonal.

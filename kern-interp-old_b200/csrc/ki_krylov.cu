@@ -33,7 +33,7 @@ constexpr int kMvThreads = 256;
 // the blocks fill the GPU: a source's values are loaded from shared memory
 // once for both, as 16-byte loads, and two independent chains per source keep
 // the FP64 pipe, which bounds this kernel, full.  65,536 Stokes dofs: 1.31 ms
-// -> 1.17 ms with the two targets and the zero test off that pipe; the pipe's
+// -> 1.15 ms with the two targets and the zero test off that pipe; the pipe's
 // own time for 17 operations per pair is 1.10 ms (one warp instruction in
 // 2.25 cycles per scheduler).
 template <int PDE, int H>
@@ -91,13 +91,17 @@ __global__ void __launch_bounds__(kMvThreads / H)
       }
     }
     __syncthreads();
-#pragma unroll 4
-    for (int q = 0; q < kMvThreads; q++) {
-      const double2 p = spos.get(q), a = samp.get(q);
-      const double2 d = PDE == kStokes ? sden.get(q) : make_double2(0.0, 0.0);
+    const int cnt = min(kMvThreads, (s1 - base + 3) & ~3);  // (the padding past it is not summed)
+#pragma unroll 1
+    for (int q4 = 0; q4 < cnt; q4 += 4) {
 #pragma unroll
-      for (int h = 0; h < H; h++)
-        pair_sum<PDE>(tx[h], ty[h], tnx[h], tny[h], p.x, p.y, a.x, a.y, d.x, d.y, y0[h], y1[h]);
+      for (int q = q4; q < q4 + 4; q++) {
+        const double2 p = spos.get(q), a = samp.get(q);
+        const double2 d = PDE == kStokes ? sden.get(q) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int h = 0; h < H; h++)
+          pair_sum<PDE>(tx[h], ty[h], tnx[h], tny[h], p.x, p.y, a.x, a.y, d.x, d.y, y0[h], y1[h]);
+      }
     }
   }
 #pragma unroll
@@ -571,21 +575,13 @@ int matvec_splits(int pde, const std::vector<int>& seg, int num_sms) {
     tiles.push_back((seg[p + 1] - seg[p] + kMvThreads - 1) / kMvThreads);
     most = std::max(most, tiles.back());
   }
-  const bool one = tiles.size() == 1;
   int best = 1;
   double best_t = 1e300;
   for (int S = 1; S <= std::min(most, kMaxMatvecSplits); S++) {  // >= 256 sources each
-    double t;
-    if (one) {
-      // ~ waves x (sources per split): ceil(blocks / slots) / S
-      const long long blocks = static_cast<long long>(most) * S;
-      t = static_cast<double>((blocks + slots - 1) / slots) / S;
-    } else {
-      // in source tiles; a block itself costs about a third of one
-      double work = 0.0;
-      for (int n : tiles) work += n * (n + S / 3.0);
-      t = work / slots + (most + S - 1) / S + 1.0 / 3.0;
-    }
+    // in source tiles; a block itself costs about a third of one
+    double work = 0.0;
+    for (int n : tiles) work += n * (n + S / 3.0);
+    const double t = work / slots + (most + S - 1) / S;
     if (t < best_t * (1.0 - 1e-9)) {
       best_t = t;
       best = S;
@@ -633,7 +629,7 @@ cudaError_t launch_fast_matvec(int pde, const Node* nodes, const MvTile* tiles, 
   if (splits < 1 || splits > kMaxMatvecSplits) return cudaErrorInvalidValue;
   double* part_rank1 = part + static_cast<long long>(splits) * n_dofs;
   count_launches(nb ? 3 : 2);
-  if (sum_targets(ntiles, num_sms) == 1) {
+  if (sum_targets(ntiles, num_sms, kOperatorSingle) == 1) {
     launch_partial<1>(pde, nodes, tiles, ntiles, n_dofs, x, part, part_rank1, s);
   } else {
     launch_partial<2>(pde, nodes, tiles, ntiles, n_dofs, x, part, part_rank1, s);

@@ -1,6 +1,6 @@
 """Operator and domain sums on both sides of the line between one target per
-thread and two (1,184 blocks of 256 targets on 148 SMs), against sums of the
-exact entries: within 8 units in the last place per term, relative to the
+thread and two (on 148 SMs: 148 blocks of 256 targets for the operator, 296
+for the domain sums), and of full launches, against sums of the exact entries: within 8 units in the last place per term, relative to the
 largest."""
 import numpy as np
 import pytest
@@ -15,7 +15,7 @@ MAKE = {"laplace": lambda n: G.star_case(n=n, n_targets=4),
 
 
 @pytest.mark.parametrize("pde", list(MAKE))
-@pytest.mark.parametrize("n", [4096, 8704, 8960, 16384])
+@pytest.mark.parametrize("n", [3071, 3072, 3073, 4096, 8704, 8960, 16384])
 def test_operator(pde, n):
     import torch
     s = kinterp.Solver(MAKE[pde](n), id_tol=1e-3)
@@ -29,7 +29,7 @@ def test_operator(pde, n):
 
 
 @pytest.mark.parametrize("pde", list(MAKE))
-@pytest.mark.parametrize("nt", [592 * 256, 592 * 256 + 1])
+@pytest.mark.parametrize("nt", [148 * 256, 148 * 256 + 1, 592 * 256, 592 * 256 + 1])
 def test_domain(pde, nt):
     pr = MAKE[pde](1000)  # two splits of the sources
     s = kinterp.Solver(pr, id_tol=1e-3)
